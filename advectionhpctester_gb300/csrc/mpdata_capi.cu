@@ -417,7 +417,8 @@ int mpdata_ws_create(const mpdata_grid* grid, const mpdata_opts* opts, void** ws
   w->fz_extrema = false;
   size_t elems = w->ncell * NSCRATCH + w->nhi;
   if (w->fused) {
-    w->fz_kchunk = fused_kchunk(geo_of(*grid));
+    const Geo fg = geo_of(*grid);
+    fused_kchunk(&fg, 1, &w->fz_kchunk);
     const size_t fz = fused_arena_elems(geo_of(*grid), &w->fz_px);
     if (fz > elems) elems = fz;
   }
@@ -676,6 +677,7 @@ struct Batch {
   // all of them; the others run on the tile kernels above
   std::vector<int> fzi;            // index in the fused table, or -1
   int nfz;
+  std::vector<int> fz_kchunk;      // z-march chunk of each fused problem
   std::vector<FusedArgs> fz_args;  // host image of the fused table
   void* d_fz;
   void* d_maps;                    // one tensor map per fused problem
@@ -827,7 +829,7 @@ void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
       F.arena = base + b->foff[p];
       fused_arena_elems(P.g, &F.px);
       F.fs = (long)F.px * P.g.mp * P.g.lp;
-      F.kchunk = fused_kchunk(P.g);
+      F.kchunk = b->fz_kchunk[f];
       F.err = b->d_err;
       F.tmap = nullptr;
       b->fz_args[f] = fused_args(F);
@@ -949,6 +951,11 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
     // fused problems: argument table, tensor maps of their arenas, work items
     std::vector<CUtensorMap> maps(b->nfz);
     std::vector<unsigned long long> up, rest;
+    std::vector<Geo> geos;
+    for (int p = 0; p < nprob; p++)
+      if (b->fzi[p] >= 0) geos.push_back(geo_of(grid_of(b, p)));
+    b->fz_kchunk.resize(b->nfz);
+    fused_kchunk(geos.data(), b->nfz, b->fz_kchunk.data());
     for (int p = 0; p < nprob && ok; p++) {
       const int f = b->fzi[p];
       if (f < 0) continue;
@@ -956,7 +963,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       int px = 0;
       fused_arena_elems(g, &px);
       ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], px, g) == 0;
-      fused_items(g, fused_kchunk(g), f, up, rest);
+      fused_items(g, b->fz_kchunk[f], f, up, rest);
     }
     ok = ok && up.size() < 0x7fffffffu && rest.size() < 0x7fffffffu && fused_init() == 0 &&
          cudaMalloc(&b->d_fz, b->nfz * sizeof(FusedArgs)) == cudaSuccess &&

@@ -48,8 +48,9 @@ bool fused_eligible(const Geo& g, int precision, int gauge, int nonos, int iord,
 size_t fused_arena_elems(const Geo& g, int* px);
 // Encodes the arena's tensor map (box 40 x 12 x 1 x 1).  0 on success.
 int fused_make_tmap(CUtensorMap* map, float* arena, int px, const Geo& g);
-// Planes per block of the z-march for this grid (MPDATA_FUSED_KCHUNK overrides).
-int fused_kchunk(const Geo& g);
+// Planes per block of the z-march for each of the n grids that one launch
+// covers (MPDATA_FUSED_KCHUNK overrides).
+void fused_kchunk(const Geo* g, int n, int* kchunk);
 // One step; on return *mx_field / *mn_field name the arena fields that hold
 // the running extrema of the step (-1 when iord = 2 keeps none).
 int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int* mx_field, int* mn_field);
