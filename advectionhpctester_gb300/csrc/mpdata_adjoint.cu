@@ -170,8 +170,8 @@ __device__ __forceinline__ void ka_update_cell(const Prob<R>& P, const AdjArr<R>
   const R ln = A.lam.ld(i, j, k);
   const R rh = P.rhr.ld(i, j, k);
   const R lt = rh * ln;                 // d x_new / d t, t = q - D/h
-  A.lxant.at(i, j, k) = lt / rh;        // q = xant/rhr
-  const R lD = -lt / P.h.ld(i, j, k);
+  A.lxant.at(i, j, k) = quot(lt, rh);        // q = xant/rhr
+  const R lD = quot(-lt, P.h.ld(i, j, k));
   fx_add<R, false, IN>(g, A.lw1, i + 1, j, k, lD);
   fx_add<R, false, IN>(g, A.lw1, i, j, k, -lD);
   fy_add<R, false, IN>(g, A.lw2, i, j + 1, k, lD);
@@ -325,7 +325,7 @@ __device__ __forceinline__ void ka_bounds_cell(const Prob<R>& P, const AdjArr<R>
     const R ep = Eps<R>::v;
     const R Dp = pn(e1) + pp(w1) + pn(e2) + pp(w2) + pn(e3) + pp(w3) + ep;
     const R Dn = pp(e1) + pn(w1) + pp(e2) + pn(w2) + pp(e3) + pn(w3) + ep;
-    const R rp = R(1) / Dp, rn = R(1) / Dn;
+    const R rp = quot(R(1), Dp), rn = quot(R(1), Dn);
     lnum_p = lcp * hc * rp;
     lnum_n = lcn * hc * rn;
     lDp = -(lnum_p * (ma.v - x)) * rp;
@@ -647,12 +647,12 @@ __device__ __forceinline__ VcTerm<R> vcorra_adj(const Geo& g, const Arr<R>& X, c
   const R y1 = (fabs(p1) + fabs(p2)) - (fabs(m1) + fabs(m2));
   const R y2 = fabs(p1) + fabs(p2) + fabs(m1) + fabs(m2) + Eps<R>::v;
   const R t = -R(0.125) * hm;
-  const R dy1 = t * a * b / y2, dy2 = -t * a * b * y1 / (y2 * y2);
+  const R dy1 = quot(t * a * b, y2), dy2 = quot(-t * a * b * y1, y2 * y2);
   xr_add<R, IN>(g, LX, pi1, pj1, pk1, lv * (dy1 + dy2) * dabs(p1));
   xr_add<R, IN>(g, LX, pi2, pj2, pk2, lv * (dy1 + dy2) * dabs(p2));
   xr_add<R, IN>(g, LX, mi1, mj1, mk1, lv * (dy2 - dy1) * dabs(m1));
   xr_add<R, IN>(g, LX, mi2, mj2, mk2, lv * (dy2 - dy1) * dabs(m2));
-  return VcTerm<R>{lv * t * a * y1 / y2, lv * t * b * y1 / y2};
+  return VcTerm<R>{quot(lv * t * a * y1, y2), quot(lv * t * b * y1, y2)};
 }
 
 // pseudo-velocity: f*ns = donor(xl, xr, v) first, then
@@ -667,7 +667,7 @@ __device__ __forceinline__ void ka_pseudo_std_cell(const Prob<R>& P, const AdjAr
   const Arr<R>& U3 = AIN ? P.u3 : P.w3;
   const R ep = Eps<R>::v;
   const bool zt = IN || g.bz || (k > 1 && k < g.lp);
-  addat(A.lxant, i, j, k, A.lq.ld(i, j, k) / P.rhr.ld(i, j, k));
+  addat(A.lxant, i, j, k, quot(A.lq.ld(i, j, k), P.rhr.ld(i, j, k)));
 #define XX(a, b, c) xr<R, IN>(g, X, (a), (b), (c))
 #define LX(a, b, c, v) xr_add<R, IN>(g, A.lxant, (a), (b), (c), (v))
 #define AX(f, b, c) fx<R, AIN, IN>(g, U1, (f), (b), (c))
@@ -682,9 +682,9 @@ __device__ __forceinline__ void ka_pseudo_std_cell(const Prob<R>& P, const AdjAr
   LX(i, j, k, -lf * pn(v));                                                                         \
   const R lv = LV.ld(i, j, k) + lf * (dpp(v) * xl - dpn(v) * xrr);                                  \
   const R K = fabs(a) - a * a * hm, N = fabs(xrr) - fabs(xl), Dd = fabs(xrr) + fabs(xl) + ep;       \
-  R la = lv * (dabs(a) - R(2) * a * hm) * N / Dd;                                                   \
-  LX(i, j, k, lv * K * dabs(xrr) * (Dd - N) / (Dd * Dd));                                           \
-  LX(XLI, XLJ, XLK, -lv * K * dabs(xl) * (Dd + N) / (Dd * Dd));
+  R la = quot(lv * (dabs(a) - R(2) * a * hm) * N, Dd);                                              \
+  LX(i, j, k, quot(lv * K * dabs(xrr) * (Dd - N), Dd * Dd));                                        \
+  LX(XLI, XLJ, XLK, quot(-lv * K * dabs(xl) * (Dd + N), Dd * Dd));
   if (IN || g.bx || i > 1) {
     FACE_HEAD(A.lv1, A.lf1, P.v1, (fx<R, AIN, IN>(g, U1, i, j, k)), P.hmx, i - 1, j, k)
     {
@@ -885,9 +885,9 @@ __global__ void __launch_bounds__(128) ka_rho_out(const Prob<R> P, const Arr<R> 
   const R pe = P.pexe.ld(i, j, k), ra = P.x_incomp.ld(i, j, k);
   const R a_xc = lxc.p ? lxc.ld(i, j, k) : R(0), a_p1 = lp1.p ? lp1.ld(i, j, k) : R(0),
           a_p2 = lp2.p ? lp2.ld(i, j, k) : R(0), a_rh = lrh.p ? lrh.ld(i, j, k) : R(0);
-  const R l_xc = a_xc + a_p1 * pe + a_p2 - a_rh * (ra / xc) / xc;
+  const R l_xc = a_xc + a_p1 * pe + a_p2 - quot(a_rh * quot(ra, xc), xc);
   lam.at(i, j, k) = lam.ld(i, j, k) + l_xc * h;
-  g_xinc.at(i, j, k) = a_rh / xc;
+  g_xinc.at(i, j, k) = quot(a_rh, xc);
   g_pexe.at(i, j, k) = a_p1 * xc;
 }
 

@@ -127,11 +127,11 @@ __device__ __forceinline__ bool warp_on_grid(const Geo& g, int i, int j) {
 // ka = |a|-a*a*hm, vcorra with bc = (0.125*a)*b.  Same operations, same order.
 template <class R>
 __device__ __forceinline__ R vdyfa_k(R x1, R x2, R ka, R ep) {
-  return ka * (fabs(x2) - fabs(x1)) / (fabs(x2) + fabs(x1) + ep);
+  return quot(ka * (fabs(x2) - fabs(x1)), fabs(x2) + fabs(x1) + ep);
 }
 template <bool U, class R>
 __device__ __forceinline__ R vcorra_b(R bc, R y1, R y2, R hm) {
-  return -(hmul<U>(bc * y1, hm) / y2);
+  return -quot(hmul<U>(bc * y1, hm), y2);
 }
 
 // True when hmx, hmy and hmz are exactly 1 at every cell of the warp (FP64
@@ -717,8 +717,8 @@ __device__ __forceinline__ RatioOps<R> bounds_body(const Prob<R>& P, int i, int 
     dn = pp(e1) + pn(w1) + pp(e2) + pn(w2) + pp(e3) + pn(w3) + ep;
   }
   if (CLM == 2) return {np_, dp, nn, dn};
-  P.cp.at(i, j, k) = CLM ? lim_ratio(np_, dp) : np_ / dp;
-  P.cn.at(i, j, k) = CLM ? lim_ratio(nn, dn) : nn / dn;
+  P.cp.at(i, j, k) = CLM ? lim_ratio(np_, dp) : quot(np_, dp);
+  P.cn.at(i, j, k) = CLM ? lim_ratio(nn, dn) : quot(nn, dn);
   return {};
 }
 
@@ -763,7 +763,7 @@ __device__ __forceinline__ void block_ratios(const Prob<R>& P, int i, int j, int
   // of the packed list skip the division
   for (int it = tid; it < total; it += nt) {
     const R n = s_n[it], d = s_d[it];
-    if (!ratio_zero(n, d)) s_n[it] = n / d;
+    if (!ratio_zero(n, d)) s_n[it] = quot(n, d);
   }
   __syncthreads();
   if (valid) {
@@ -910,7 +910,7 @@ __device__ __forceinline__ void rho_out_body(const Prob<R>& P, int i, int j, int
   P.x_incomp.at(i, j, k) = xc;
   P.pexr1.at(i, j, k) = xc * P.pexe.ld(i, j, k);
   P.pexr2.at(i, j, k) = xc;
-  P.rhr_out.at(i, j, k) = P.rhoadv.ld(i, j, k) / xc;
+  P.rhr_out.at(i, j, k) = quot(P.rhoadv.ld(i, j, k), xc);
   P.u1.at(i, j, k) = P.f1.ld(i, j, k) + (LINER ? R(0) : fx<R, false>(g, P.w1, i, j, k));
   P.u2.at(i, j, k) = P.f2.ld(i, j, k) + (LINER ? R(0) : fy<R, false>(g, P.w2, i, j, k));
   P.u3.at(i, j, k) = P.f3.ld(i, j, k) + (LINER ? R(0) : fz<R, false>(g, P.w3, i, j, k));
