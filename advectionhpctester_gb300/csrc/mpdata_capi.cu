@@ -175,6 +175,9 @@ int ws_step(Workspace* w, const Prob<R>& P, Prof* prof, cudaStream_t s) {
     if (w->fused) {
       FusedPlan F;
       F.g = P.g;
+      F.cls = fused_class(P.g, !P.stdf);
+      F.bcx = P.bcx;
+      F.bcy = P.bcy;
       F.psi = P.psi;
       F.u1 = P.u1;
       F.u2 = P.u2;
@@ -681,9 +684,8 @@ struct Batch {
   std::vector<FusedArgs> fz_args;  // host image of the fused table
   void* d_fz;
   void* d_maps;                    // one tensor map per fused problem
-  unsigned long long* d_items_up;  // work items of the upwind+pseudo kernel
-  unsigned long long* d_items;     // ... of the other fused kernels
-  int n_items_up, n_items;
+  unsigned long long* d_items;     // work items: per class, the upwind+pseudo kernel's, then the others'
+  FusedItems fz_items[FZ_NCLASS];
   int* d_err;
 };
 
@@ -792,7 +794,7 @@ int batch_run(Batch* b, int halo, Prof* prof, cudaStream_t s) {
   }
   if (halo && b->nfz &&
       run_batch_fused(static_cast<const FusedArgs*>(b->d_fz), static_cast<const CUtensorMap*>(b->d_maps),
-                      b->d_items_up, b->n_items_up, b->d_items, b->n_items, b->iord, prof, s))
+                      b->fz_items, b->iord, prof, s))
     return MPDATA_E_CUDA;
   return MPDATA_OK;
 }
@@ -820,6 +822,9 @@ void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
     if (f >= 0) {
       FusedPlan F;
       F.g = P.g;
+      F.cls = fused_class(P.g, !P.stdf);
+      F.bcx = P.bcx;
+      F.bcy = P.bcy;
       F.psi = P.psi;
       F.u1 = P.u1;
       F.u2 = P.u2;
@@ -879,8 +884,8 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   b->fzi.assign(nprob, -1);
   b->nfz = 0;
   b->d_fz = b->d_maps = nullptr;
-  b->d_items_up = b->d_items = nullptr;
-  b->n_items_up = b->n_items = 0;
+  b->d_items = nullptr;
+  for (FusedItems& I : b->fz_items) I = FusedItems{nullptr, nullptr, 0, 0};
   b->d_err = nullptr;
   size_t off = 0;
   for (int p = 0; p < nprob; p++) {
@@ -918,7 +923,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
     }
     for (int p = 0; p < nprob; p++) {
       const int o = b->owner[p];
-      b->gv[p] = (iord >= 2 && members[o] >= 2) ? forms[o] : 0;
+      b->gv[p] = (iord >= 2 && members[o] >= 2 && b->fzi[p] < 0) ? forms[o] : 0;
     }
   }
   for (int p = 0; p < nprob; p++)
@@ -950,7 +955,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   if (ok && b->nfz) {
     // fused problems: argument table, tensor maps of their arenas, work items
     std::vector<CUtensorMap> maps(b->nfz);
-    std::vector<unsigned long long> up, rest;
+    std::vector<unsigned long long> up[FZ_NCLASS], rest[FZ_NCLASS];
     std::vector<Geo> geos;
     for (int p = 0; p < nprob; p++)
       if (b->fzi[p] >= 0) geos.push_back(geo_of(grid_of(b, p)));
@@ -963,22 +968,29 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       int px = 0;
       fused_arena_elems(g, &px);
       ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], px, g) == 0;
-      fused_items(g, b->fz_kchunk[f], f, up, rest);
+      const int c = fused_class(g, probs[p].gauge);
+      fused_items(g, b->fz_kchunk[f], f, up[c], rest[c]);
     }
-    ok = ok && up.size() < 0x7fffffffu && rest.size() < 0x7fffffffu && fused_init() == 0 &&
+    std::vector<unsigned long long> all;
+    for (int c = 0; c < FZ_NCLASS; c++) {
+      all.insert(all.end(), up[c].begin(), up[c].end());
+      all.insert(all.end(), rest[c].begin(), rest[c].end());
+    }
+    ok = ok && all.size() < 0x7fffffffu && fused_init() == 0 &&
          cudaMalloc(&b->d_fz, b->nfz * sizeof(FusedArgs)) == cudaSuccess &&
          cudaMalloc(&b->d_maps, b->nfz * sizeof(CUtensorMap)) == cudaSuccess &&
-         cudaMalloc(&b->d_items_up, up.size() * sizeof(unsigned long long)) == cudaSuccess &&
-         cudaMalloc(&b->d_items, rest.size() * sizeof(unsigned long long)) == cudaSuccess &&
+         cudaMalloc(&b->d_items, all.size() * sizeof(unsigned long long)) == cudaSuccess &&
          cudaMalloc(&b->d_err, sizeof(int)) == cudaSuccess && cudaMemset(b->d_err, 0, sizeof(int)) == cudaSuccess &&
          cudaMemcpy(b->d_maps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice) ==
              cudaSuccess &&
-         cudaMemcpy(b->d_items_up, up.data(), up.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice) ==
-             cudaSuccess &&
-         cudaMemcpy(b->d_items, rest.data(), rest.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice) ==
+         cudaMemcpy(b->d_items, all.data(), all.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice) ==
              cudaSuccess;
-    b->n_items_up = (int)up.size();
-    b->n_items = (int)rest.size();
+    size_t at = 0;
+    for (int c = 0; c < FZ_NCLASS; c++) {
+      b->fz_items[c] = FusedItems{b->d_items + at, b->d_items + at + up[c].size(), (int)up[c].size(),
+                                  (int)rest[c].size()};
+      at += up[c].size() + rest[c].size();
+    }
   }
   if (ok) {
     // default shape, or the tuned one for this batch signature
@@ -1014,7 +1026,6 @@ int mpdata_batch_destroy(void* batch) {
   cudaFree(b->d_table);
   cudaFree(b->d_fz);
   cudaFree(b->d_maps);
-  cudaFree(b->d_items_up);
   cudaFree(b->d_items);
   cudaFree(b->d_err);
   cudaError_t e = cudaFree(b->mem);

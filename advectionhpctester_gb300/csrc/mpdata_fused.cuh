@@ -16,11 +16,17 @@ namespace mpdata {
 enum FusedField { FZ_XIN = 0, FZ_X0, FZ_X1, FZ_V1, FZ_V2, FZ_V3, FZ_W1, FZ_W2, FZ_W3, FZ_MX0, FZ_MN0, FZ_MX1,
                   FZ_MN1, FZ_NF };
 
+// The kernel instantiations a problem runs on: the gauge form on a grid that is
+// periodic on every axis (wraps only), the gauge form with open or wall axes,
+// the standard form on any grid.
+enum FusedClass { FZ_PERIODIC = 0, FZ_WALL, FZ_STD, FZ_NCLASS };
+
 // Arguments of the fused kernels for one problem: caller arrays, the arena,
 // the z-march chunk, and the arena fields of the current pass.
 struct FusedArgs {
   Geo g;
   Arr<float> psi, u1, u2, u3, h, rhr;
+  const float *bcx, *bcy;  // Dirichlet halo values of psi on open x and y walls
   float* arena;
   int px;
   long fs;
@@ -32,7 +38,9 @@ struct FusedArgs {
 
 struct FusedPlan {
   Geo g;
+  FusedClass cls;
   Arr<float> psi, u1, u2, u3, h, rhr;  // caller arrays
+  const float *bcx, *bcy;
   float* arena;
   int px;       // arena row pitch (elements)
   long fs;      // elements per arena field
@@ -41,9 +49,10 @@ struct FusedPlan {
   const CUtensorMap* tmap;  // one 4-D map over the arena (x, y, z, field)
 };
 
-// Whether a step takes the fused path: FP32, infinite gauge, nonoscillatory,
-// iord >= 2, every axis periodic, not the density step.
+// Whether a step takes the fused path: FP32, nonoscillatory, iord >= 2, not the
+// density step.
 bool fused_eligible(const Geo& g, int precision, int gauge, int nonos, int iord, int rho);
+FusedClass fused_class(const Geo& g, int gauge);
 // Arena geometry: the row pitch and the total elements of the FZ_NF fields.
 size_t fused_arena_elems(const Geo& g, int* px);
 // Encodes the arena's tensor map (box 40 x 12 x 1 x 1).  0 on success.
@@ -58,14 +67,19 @@ int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int
 // Batches.  Each problem of the fused table gets work items (a tile of the
 // upwind+pseudo kernel's height, or of the other kernels' height, and a z
 // chunk) packed as problem | tile x << 16 | tile y << 32 | chunk << 48; one
-// launch per fused kernel then covers every problem.
+// launch per fused kernel and class then covers every problem.
 FusedArgs fused_args(const FusedPlan& F);
 void fused_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& up,
                  std::vector<unsigned long long>& rest);
 int fused_init();
-// One step of every problem of the table (device arrays: args, tensor maps,
-// the two item lists).
-int run_batch_fused(const FusedArgs* probs, const CUtensorMap* maps, const unsigned long long* items_up, int n_up,
-                    const unsigned long long* items, int n, int iord, Prof* prof, cudaStream_t s);
+// The device work lists of one class.
+struct FusedItems {
+  const unsigned long long *up, *rest;
+  int n_up, n;
+};
+// One step of every problem of the table (device arrays: args, tensor maps;
+// items: FZ_NCLASS lists, empty ones with n = 0).
+int run_batch_fused(const FusedArgs* probs, const CUtensorMap* maps, const FusedItems* items, int iord, Prof* prof,
+                    cudaStream_t s);
 
 }  // namespace mpdata
