@@ -99,7 +99,7 @@ struct Workspace {
   // fused single-precision path (periodic gauge grids): its arena shares
   // `mem` with the stage path's scratch, which it never needs at the same time
   bool fused;
-  int fz_px, fz_kchunk;
+  int fz_kchunk;
   int fz_mx, fz_mn;    // arena fields holding the last fused step's extrema (-1: none)
   bool fz_extrema;     // the last step ran fused: the extrema live in the arena
   alignas(64) CUtensorMap fz_map;
@@ -185,8 +185,6 @@ int ws_step(Workspace* w, const Prob<R>& P, Prof* prof, cudaStream_t s) {
       F.h = P.h;
       F.rhr = P.rhr;
       F.arena = static_cast<float*>(w->mem);
-      F.px = w->fz_px;
-      F.fs = (long)w->fz_px * w->g.mp * w->g.lp;
       F.kchunk = w->fz_kchunk;
       F.err = w->d_err;
       F.tmap = &w->fz_map;
@@ -384,9 +382,9 @@ int count_violations(Workspace* w, const void* psi, double tol, unsigned long lo
   const Prob<R> P = make_prob<R>(w->g, w->o.gauge, x, x, x, x, x, x, nullptr, nullptr, base, w->ncell,
                                  base + (size_t)NFIELD * w->ncell, 1);
   if (w->fz_extrema && w->fz_mx >= 0) {  // the last step ran fused: its extrema are arena fields
-    const long fs = (long)w->fz_px * w->g.mp * w->g.lp;
-    const Arr<R> mx{base + (size_t)w->fz_mx * fs, w->fz_px, w->fz_px * w->g.mp};
-    const Arr<R> mn{base + (size_t)w->fz_mn * fs, w->fz_px, w->fz_px * w->g.mp};
+    const Arr<float> fx = fused_view(static_cast<float*>(w->mem), w->fz_mx, P.g),
+                     fn = fused_view(static_cast<float*>(w->mem), w->fz_mn, P.g);
+    const Arr<R> mx{reinterpret_cast<R*>(fx.p), fx.sy, fx.sz}, mn{reinterpret_cast<R*>(fn.p), fn.sy, fn.sz};
     return run_bound_violations<R>(P.g, P.psi, mx, mn, tol, d, s) ? MPDATA_E_CUDA : MPDATA_OK;
   }
   return run_bound_violations<R>(P.g, P.psi, P.mx, P.mn, tol, d, s) ? MPDATA_E_CUDA : MPDATA_OK;
@@ -422,7 +420,7 @@ int mpdata_ws_create(const mpdata_grid* grid, const mpdata_opts* opts, void** ws
   if (w->fused) {
     const Geo fg = geo_of(*grid);
     fused_kchunk(&fg, 1, &w->fz_kchunk);
-    const size_t fz = fused_arena_elems(geo_of(*grid), &w->fz_px);
+    const size_t fz = fused_arena(geo_of(*grid)).elems;
     if (fz > elems) elems = fz;
   }
   if (cudaMalloc(&w->mem, elems * w->elem) != cudaSuccess) {
@@ -436,7 +434,7 @@ int mpdata_ws_create(const mpdata_grid* grid, const mpdata_opts* opts, void** ws
     delete w;
     return MPDATA_E_CUDA;
   }
-  if (w->fused && fused_make_tmap(&w->fz_map, static_cast<float*>(w->mem), w->fz_px, geo_of(*grid))) {
+  if (w->fused && fused_make_tmap(&w->fz_map, static_cast<float*>(w->mem), geo_of(*grid))) {
     cudaFree(w->mem);
     cudaFree(w->d_err);
     delete w;
@@ -684,7 +682,7 @@ struct Batch {
   std::vector<FusedArgs> fz_args;  // host image of the fused table
   void* d_fz;
   void* d_maps;                    // one tensor map per fused problem
-  unsigned long long* d_items;     // work items: per class, the upwind+pseudo kernel's, then the others'
+  unsigned long long* d_items;     // work items, class after class
   FusedItems fz_items[FZ_NCLASS];
   int* d_err;
 };
@@ -832,8 +830,6 @@ void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
       F.h = P.h;
       F.rhr = P.rhr;
       F.arena = base + b->foff[p];
-      fused_arena_elems(P.g, &F.px);
-      F.fs = (long)F.px * P.g.mp * P.g.lp;
       F.kchunk = b->fz_kchunk[f];
       F.err = b->d_err;
       F.tmap = nullptr;
@@ -885,7 +881,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   b->nfz = 0;
   b->d_fz = b->d_maps = nullptr;
   b->d_items = nullptr;
-  for (FusedItems& I : b->fz_items) I = FusedItems{nullptr, nullptr, 0, 0};
+  for (FusedItems& I : b->fz_items) I = FusedItems{nullptr, 0};
   b->d_err = nullptr;
   size_t off = 0;
   for (int p = 0; p < nprob; p++) {
@@ -909,7 +905,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
     b->owner[p] = own;
     b->foff[p] = off;
     size_t nf = (size_t)NFIELD * b->ncell[p];
-    if (b->fzi[p] >= 0) nf = std::max(nf, fused_arena_elems(geo_of(g), nullptr));
+    if (b->fzi[p] >= 0) nf = std::max(nf, fused_arena(geo_of(g)).elems);
     off += (nf + 63) / 64 * 64;  // 256-byte aligned regions (TMA wants 16)
   }
   // a group of two or more fields shares the velocity-only terms of its
@@ -955,7 +951,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   if (ok && b->nfz) {
     // fused problems: argument table, tensor maps of their arenas, work items
     std::vector<CUtensorMap> maps(b->nfz);
-    std::vector<unsigned long long> up[FZ_NCLASS], rest[FZ_NCLASS];
+    std::vector<unsigned long long> items[FZ_NCLASS];
     std::vector<Geo> geos;
     for (int p = 0; p < nprob; p++)
       if (b->fzi[p] >= 0) geos.push_back(geo_of(grid_of(b, p)));
@@ -965,17 +961,12 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       const int f = b->fzi[p];
       if (f < 0) continue;
       const Geo g = geo_of(grid_of(b, p));
-      int px = 0;
-      fused_arena_elems(g, &px);
-      ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], px, g) == 0;
+      ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], g) == 0;
       const int c = fused_class(g, probs[p].gauge);
-      fused_items(g, b->fz_kchunk[f], f, up[c], rest[c]);
+      fused_items(g, b->fz_kchunk[f], f, items[c]);
     }
     std::vector<unsigned long long> all;
-    for (int c = 0; c < FZ_NCLASS; c++) {
-      all.insert(all.end(), up[c].begin(), up[c].end());
-      all.insert(all.end(), rest[c].begin(), rest[c].end());
-    }
+    for (int c = 0; c < FZ_NCLASS; c++) all.insert(all.end(), items[c].begin(), items[c].end());
     ok = ok && all.size() < 0x7fffffffu && fused_init() == 0 &&
          cudaMalloc(&b->d_fz, b->nfz * sizeof(FusedArgs)) == cudaSuccess &&
          cudaMalloc(&b->d_maps, b->nfz * sizeof(CUtensorMap)) == cudaSuccess &&
@@ -987,9 +978,8 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
              cudaSuccess;
     size_t at = 0;
     for (int c = 0; c < FZ_NCLASS; c++) {
-      b->fz_items[c] = FusedItems{b->d_items + at, b->d_items + at + up[c].size(), (int)up[c].size(),
-                                  (int)rest[c].size()};
-      at += up[c].size() + rest[c].size();
+      b->fz_items[c] = FusedItems{b->d_items + at, (int)items[c].size()};
+      at += items[c].size();
     }
   }
   if (ok) {

@@ -8,11 +8,11 @@
 
 namespace mpdata {
 
-// Fields of the fused step's arena, each px*mp*lp floats (rows padded to a
-// multiple of 4 elements so that every row starts on a 16-byte boundary, as
-// TMA requires): the step's input field, the two ping-pong fields of the
-// passes, pseudo and limited velocities, and two ping-pong pairs of running
-// extrema.
+// Fields of the fused step's arena, each px*(mp+4)*lp floats (a halo of four
+// columns and two rows on every side; rows a multiple of 4 elements so that
+// every row starts on a 16-byte boundary, as TMA requires): the step's input
+// field, the two ping-pong fields of the passes, pseudo and limited
+// velocities, and two ping-pong pairs of running extrema.
 enum FusedField { FZ_XIN = 0, FZ_X0, FZ_X1, FZ_V1, FZ_V2, FZ_V3, FZ_W1, FZ_W2, FZ_W3, FZ_MX0, FZ_MN0, FZ_MX1,
                   FZ_MN1, FZ_NF };
 
@@ -30,6 +30,8 @@ struct FusedArgs {
   float* arena;
   int px;
   long fs;
+  int ntx, nty;                       // tiles along x and y
+  unsigned char* flags;               // per plane and tile: h and rhr all exactly 1 (written by the first kernel)
   int kchunk;
   int fin, fout;                      // pass input / output field
   int fmx_in, fmn_in, fmx_out, fmn_out;
@@ -42,8 +44,6 @@ struct FusedPlan {
   Arr<float> psi, u1, u2, u3, h, rhr;  // caller arrays
   const float *bcx, *bcy;
   float* arena;
-  int px;       // arena row pitch (elements)
-  long fs;      // elements per arena field
   int kchunk;   // planes per block of the z-march
   int* err;     // device error word (bit 1: a staging wait timed out)
   const CUtensorMap* tmap;  // one 4-D map over the arena (x, y, z, field)
@@ -53,10 +53,18 @@ struct FusedPlan {
 // density step.
 bool fused_eligible(const Geo& g, int precision, int gauge, int nonos, int iord, int rho);
 FusedClass fused_class(const Geo& g, int gauge);
-// Arena geometry: the row pitch and the total elements of the FZ_NF fields.
-size_t fused_arena_elems(const Geo& g, int* px);
-// Encodes the arena's tensor map (box 40 x 12 x 1 x 1).  0 on success.
-int fused_make_tmap(CUtensorMap* map, float* arena, int px, const Geo& g);
+// Arena geometry: row pitch, elements per field, tiles, and the total elements
+// of the FZ_NF fields and the flags.
+struct FusedArena {
+  int px, ntx, nty;
+  long fs;
+  size_t elems;
+};
+FusedArena fused_arena(const Geo& g);
+// An arena field's interior as an array view.
+Arr<float> fused_view(float* arena, int field, const Geo& g);
+// Encodes the arena's tensor map (box 72 x 20 x 1 x 1).  0 on success.
+int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g);
 // Planes per block of the z-march for each of the n grids that one launch
 // covers (MPDATA_FUSED_KCHUNK overrides).
 void fused_kchunk(const Geo* g, int n, int* kchunk);
@@ -64,18 +72,16 @@ void fused_kchunk(const Geo* g, int n, int* kchunk);
 // the running extrema of the step (-1 when iord = 2 keeps none).
 int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int* mx_field, int* mn_field);
 
-// Batches.  Each problem of the fused table gets work items (a tile of the
-// upwind+pseudo kernel's height, or of the other kernels' height, and a z
+// Batches.  Each problem of the fused table gets work items (a tile and a z
 // chunk) packed as problem | tile x << 16 | tile y << 32 | chunk << 48; one
 // launch per fused kernel and class then covers every problem.
 FusedArgs fused_args(const FusedPlan& F);
-void fused_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& up,
-                 std::vector<unsigned long long>& rest);
+void fused_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& items);
 int fused_init();
-// The device work lists of one class.
+// The device work list of one class.
 struct FusedItems {
-  const unsigned long long *up, *rest;
-  int n_up, n;
+  const unsigned long long* items;
+  int n;
 };
 // One step of every problem of the table (device arrays: args, tensor maps;
 // items: FZ_NCLASS lists, empty ones with n = 0).

@@ -2,8 +2,8 @@
 form, against the FP32 oracle and the stage path, bit for bit, psi's halo
 included.
 
-The sizes put the walls everywhere a tile of 32x8 (32x16) cells and a z chunk
-can meet them: inside a tile, on its edge, one column or row past it, tiles
+The sizes put the walls everywhere a tile of 64x12 cells and a z chunk can meet
+them: inside a tile, on its edge, one column or row past it, tiles
 whose boxes come in by TMA between wall tiles, grids of two cells, and z
 chunks of one plane.
 """
@@ -47,7 +47,8 @@ def same_bits(a, b):
     np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
 
 
-SIZES = [(200, 96, 24), (33, 17, 9), (37, 23, 5), (64, 16, 3), (65, 9, 2), (2, 2, 2), (32, 8, 1)]
+SIZES = [(200, 96, 24), (33, 17, 9), (37, 23, 5), (64, 12, 3), (65, 13, 2), (129, 25, 3), (127, 24, 2), (2, 2, 2),
+         (32, 8, 1)]
 BCS = [(0, 0, 0), (0, 1, 1), (1, 0, 1), (1, 1, 0), (1, 1, 1)]
 
 
