@@ -797,8 +797,10 @@ int batch_run(Batch* b, int halo, Prof* prof, cudaStream_t s) {
   return MPDATA_OK;
 }
 
+// The host image of problem p's descriptors; true when it changed (an equal one
+// needs no upload).
 template <class R>
-void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, const void* u3, const void* h,
+bool write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, const void* u3, const void* h,
                 const void* rhr, const void* bcx, const void* bcy) {
   R* base = static_cast<R*>(b->mem);
   const mpdata_grid g = grid_of(b, p);
@@ -814,7 +816,9 @@ void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
   }
   if (P.gv & 2)
     for (int s = 0; s < NGVS; s++) P.gvs[s] = scratch_view<R>(gbase + (size_t)s * b->ncell[p], P.g);
-  memcpy(b->table.data() + (size_t)p * sizeof(Prob<R>), &P, sizeof P);
+  unsigned char* const image = b->table.data() + (size_t)p * sizeof(Prob<R>);
+  bool changed = memcmp(image, &P, sizeof P) != 0;
+  memcpy(image, &P, sizeof P);
   if constexpr (sizeof(R) == 4) {
     const int f = b->fzi[p];
     if (f >= 0) {
@@ -833,9 +837,12 @@ void write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
       F.kchunk = b->fz_kchunk[f];
       F.err = b->d_err;
       F.tmap = nullptr;
-      b->fz_args[f] = fused_args(F);
+      const FusedArgs A = fused_args(F);
+      changed = changed || memcmp(&b->fz_args[f], &A, sizeof A) != 0;
+      b->fz_args[f] = A;
     }
   }
+  return changed;
 }
 
 // tuned block shapes per (precision, iord, nonos, cells), shared by batches
@@ -1030,10 +1037,10 @@ int mpdata_batch_set(void* batch, int prob, void* psi, const void* u1, const voi
   if (prob < 0 || prob >= b->nprob) return MPDATA_E_DIMS;
   if (!psi || !u1 || !u2 || !u3 || !h || !rhr) return MPDATA_E_NULL;
   if ((!b->pr[prob].ibcx && !bcx) || (!b->pr[prob].ibcy && !bcy)) return MPDATA_E_NULL;
-  if (b->precision == 64) write_prob<double>(b, prob, psi, u1, u2, u3, h, rhr, bcx, bcy);
-  else write_prob<float>(b, prob, psi, u1, u2, u3, h, rhr, bcx, bcy);
+  const bool changed = b->precision == 64 ? write_prob<double>(b, prob, psi, u1, u2, u3, h, rhr, bcx, bcy)
+                                          : write_prob<float>(b, prob, psi, u1, u2, u3, h, rhr, bcx, bcy);
+  if (changed || !b->given[prob]) b->dirty = true;
   b->given[prob] = 1;
-  b->dirty = true;
   return MPDATA_OK;
 }
 

@@ -65,6 +65,10 @@ def _is_fortran(t):
 def _ptr(t, dtype, shape=None, name="array"):
     if t is None:
         return None
+    # the usual case in few calls: a step makes up to ten of these checks
+    if shape is not None and len(shape) == 3 and t.dtype == dtype and t.is_cuda and t.shape == shape and \
+            t.stride() == (1, shape[0], shape[0] * shape[1]):
+        return t.data_ptr()
     if not t.is_cuda:
         raise ValueError("%s must be a CUDA tensor" % name)
     if t.dtype != dtype:
@@ -280,13 +284,20 @@ class Batch:
         self._keep = {}
 
     def set(self, p, psi, u1, u2, u3, h, rhr, bcx=None, bcy=None):
+        self._set(p, psi, (u1, u2, u3, h, rhr), self._velocity(p, u1, u2, u3, h, rhr), bcx, bcy)
+
+    def _velocity(self, p, u1, u2, u3, h, rhr):
         s, d = self.shapes[p], self.dtype
-        check(self.lib.mpdata_batch_set(self.handle, p, _ptr(psi, d, s["psi"], "psi"), _ptr(u1, d, s["u1"], "u1"),
-                                        _ptr(u2, d, s["u2"], "u2"), _ptr(u3, d, s["u3"], "u3"),
-                                        _ptr(h, d, s["psi"], "h"), _ptr(rhr, d, s["psi"], "rhr"),
+        return (_ptr(u1, d, s["u1"], "u1"), _ptr(u2, d, s["u2"], "u2"), _ptr(u3, d, s["u3"], "u3"),
+                _ptr(h, d, s["psi"], "h"), _ptr(rhr, d, s["psi"], "rhr"))
+
+    def _set(self, p, psi, velocity, ptrs, bcx, bcy):
+        """Problem p with the velocity and densities whose checked pointers are ptrs."""
+        s, d = self.shapes[p], self.dtype
+        check(self.lib.mpdata_batch_set(self.handle, p, _ptr(psi, d, s["psi"], "psi"), *ptrs,
                                         _ptr(bcx, d, s["bcx"], "bcx"), _ptr(bcy, d, s["bcy"], "bcy")),
               "mpdata_batch_set")
-        self._keep[p] = (psi, u1, u2, u3, h, rhr, bcx, bcy)  # keep the tensors alive
+        self._keep[p] = (psi, velocity, bcx, bcy)  # keep the tensors alive
 
     def step(self, stream=None):
         check(self.lib.mpdata_batch_step(self.handle, _stream(stream)), "mpdata_batch_step")
@@ -377,9 +388,11 @@ def ce_advection(mpdata_alg_choice, liner, ipoles, ibcx, ibcy, ibcz, np_, mp, lp
         probs = [dict(np=np_, mp=mp, lp=lp, ibcx=ibcx, ibcy=ibcy, ibcz=ibcz, gauge=f, velocity_group=0)
                  for f in forms]
         b = _ce_cache[key] = Batch(probs, ih=ih, iord=iord, nonos=1, precision=prec)
+    velocity = (uadv, vadv, wadv, rhoadv, rhr)  # one grid: checked once for every field
+    ptrs = b._velocity(0, *velocity)
     for p, n in enumerate(names):
         x, x_lr, x_bt = fields[n]
-        b.set(p, x, uadv, vadv, wadv, rhoadv, rhr, x_lr, x_bt)
+        b._set(p, x, velocity, ptrs, x_lr, x_bt)
     b.step(stream)
 
 
