@@ -682,8 +682,8 @@ struct Batch {
   std::vector<FusedArgs> fz_args;  // host image of the fused table
   void* d_fz;
   void* d_maps;                    // one tensor map per fused problem
-  unsigned long long* d_items;     // work items, class after class
-  FusedItems fz_items[FZ_NCLASS];
+  unsigned long long* d_items;     // work items: the periodic gauge problems', then the others'
+  FusedItems fz_items[2];
   int* d_err;
 };
 
@@ -958,7 +958,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   if (ok && b->nfz) {
     // fused problems: argument table, tensor maps of their arenas, work items
     std::vector<CUtensorMap> maps(b->nfz);
-    std::vector<unsigned long long> items[FZ_NCLASS];
+    std::vector<unsigned long long> items[2], last;  // last: the lighter gauge blocks end the second list
     std::vector<Geo> geos;
     for (int p = 0; p < nprob; p++)
       if (b->fzi[p] >= 0) geos.push_back(geo_of(grid_of(b, p)));
@@ -969,11 +969,12 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       if (f < 0) continue;
       const Geo g = geo_of(grid_of(b, p));
       ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], g) == 0;
-      const int c = fused_class(g, probs[p].gauge);
-      fused_items(g, b->fz_kchunk[f], f, items[c]);
+      const FusedClass c = fused_class(g, probs[p].gauge);
+      fused_items(g, b->fz_kchunk[f], f, c == FZ_PERIODIC ? items[0] : c == FZ_STD ? items[1] : last);
     }
     std::vector<unsigned long long> all;
-    for (int c = 0; c < FZ_NCLASS; c++) all.insert(all.end(), items[c].begin(), items[c].end());
+    items[1].insert(items[1].end(), last.begin(), last.end());
+    for (int c = 0; c < 2; c++) all.insert(all.end(), items[c].begin(), items[c].end());
     ok = ok && all.size() < 0x7fffffffu && fused_init() == 0 &&
          cudaMalloc(&b->d_fz, b->nfz * sizeof(FusedArgs)) == cudaSuccess &&
          cudaMalloc(&b->d_maps, b->nfz * sizeof(CUtensorMap)) == cudaSuccess &&
@@ -984,7 +985,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
          cudaMemcpy(b->d_items, all.data(), all.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice) ==
              cudaSuccess;
     size_t at = 0;
-    for (int c = 0; c < FZ_NCLASS; c++) {
+    for (int c = 0; c < 2; c++) {
       b->fz_items[c] = FusedItems{b->d_items + at, (int)items[c].size()};
       at += items[c].size();
     }

@@ -19,13 +19,14 @@ enum FusedField { FZ_XIN = 0, FZ_X0, FZ_X1, FZ_V1, FZ_V2, FZ_V3, FZ_W1, FZ_W2, F
 // The kernel instantiations a problem runs on: the gauge form on a grid that is
 // periodic on every axis (wraps only), the gauge form with open or wall axes,
 // the standard form on any grid.
-enum FusedClass { FZ_PERIODIC = 0, FZ_WALL, FZ_STD, FZ_NCLASS };
+enum FusedClass { FZ_PERIODIC = 0, FZ_WALL, FZ_STD };
 
 // Arguments of the fused kernels for one problem: caller arrays, the arena,
 // the z-march chunk, and the arena fields of the current pass.
 struct FusedArgs {
   Geo g;
   Arr<float> psi, u1, u2, u3, h, rhr;
+  int stdf;                // the standard form
   const float *bcx, *bcy;  // Dirichlet halo values of psi on open x and y walls
   float* arena;
   int px;
@@ -74,17 +75,18 @@ int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int
 
 // Batches.  Each problem of the fused table gets work items (a tile and a z
 // chunk) packed as problem | tile x << 16 | tile y << 32 | chunk << 48; one
-// launch per fused kernel and class then covers every problem.
+// launch per fused kernel and work list (the periodic gauge problems; the others)
+// then covers every problem.
 FusedArgs fused_args(const FusedPlan& F);
 void fused_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& items);
 int fused_init();
-// The device work list of one class.
+// A device work list.
 struct FusedItems {
   const unsigned long long* items;
   int n;
 };
 // One step of every problem of the table (device arrays: args, tensor maps;
-// items: FZ_NCLASS lists, empty ones with n = 0).
+// items: the two lists, empty ones with n = 0).
 int run_batch_fused(const FusedArgs* probs, const CUtensorMap* maps, const FusedItems* items, int iord, Prof* prof,
                     cudaStream_t s);
 
