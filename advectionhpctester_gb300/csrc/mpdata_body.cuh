@@ -146,6 +146,20 @@ __device__ __forceinline__ bool warp_unit_faces(const Prob<R>& P, int i, int j, 
   }
 }
 
+// The same over the warp's cells in the grid (act), a wall's face, which nothing
+// reads, not counted.  Every lane of act calls it.
+template <class R>
+__device__ __forceinline__ bool warp_unit_faces(const Prob<R>& P, int i, int j, int k, unsigned act) {
+  if constexpr (sizeof(R) == 8) {
+    const Geo& g = P.g;
+    const bool u = (!(g.bx || i > 1) || is_one(P.hmx.ld(i, j, k))) && (!(g.by || j > 1) || is_one(P.hmy.ld(i, j, k))) &&
+                   (!(g.bz || k > 1) || is_one(P.hmz.ld(i, j, k)));
+    return __all_sync(act, u);
+  } else {
+    return false;
+  }
+}
+
 // True when h (and rhr, outside the density step) is exactly 1 at every cell
 // of the warp (FP64 only).  Bodies instantiated with U drop the products and
 // quotients by these densities: exact, as x*1 == x/1 == x.
@@ -365,12 +379,17 @@ __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int 
 #define MZ(a) cz<IN>(g, (a))
 #define QX(a) xmx<IN>(g, (a))
 #define QY(a) xmy<IN>(g, (a))
-#define S2X (PV ? P.f2.ld(MX(i - 1), j, k) + P.f2.ld(i, j, k) : VSUM_2X)
-#define S3X (PV ? P.f3.ld(MX(i - 1), j, k) + P.f3.ld(i, j, k) : VSUM_3X)
-#define S1Y (PV ? P.f1.ld(i, MY(j - 1), k) + P.f1.ld(i, j, k) : VSUM_1Y)
-#define S3Y (PV ? P.f3.ld(i, MY(j - 1), k) + P.f3.ld(i, j, k) : VSUM_3Y)
-#define S1Z (PV ? P.f1.ld(i, j, MZ(k - 1)) + P.f1.ld(i, j, k) : VSUM_1Z)
-#define S2Z (PV ? P.f2.ld(i, j, MZ(k - 1)) + P.f2.ld(i, j, k) : VSUM_2Z)
+  // where k_pairs stored the velocity pairs (the standard form's f1..f3 are its output)
+  const Arr<R>&C1 = STD ? P.w1 : P.f1, &C2 = STD ? P.w2 : P.f2, &C3 = STD ? P.w3 : P.f3;
+#define S2X (PV ? C2.ld(MX(i - 1), j, k) + C2.ld(i, j, k) : VSUM_2X)
+#define S3X (PV ? C3.ld(MX(i - 1), j, k) + C3.ld(i, j, k) : VSUM_3X)
+#define S1Y (PV ? C1.ld(i, MY(j - 1), k) + C1.ld(i, j, k) : VSUM_1Y)
+#define S3Y (PV ? C3.ld(i, MY(j - 1), k) + C3.ld(i, j, k) : VSUM_3Y)
+#define S1Z (PV ? C1.ld(i, j, MZ(k - 1)) + C1.ld(i, j, k) : VSUM_1Z)
+#define S2Z (PV ? C2.ld(i, j, MZ(k - 1)) + C2.ld(i, j, k) : VSUM_2Z)
+// the four |x| around a face: their p-pair and m-pair (stored or formed), m0, m1
+#define STD_Y1(p, pm, m0, m1) ((p) - (PS ? (pm) : (m0) + (m1)))
+#define STD_Y2(p, m0, m1) ((p) + (m0) + (m1) + ep)
   // DEFER: results held until every load is issued (see limit_form); the
   // batch kernels, whose launch bound admits 256 threads, store each face at
   // once, which keeps their register count (and occupancy) lower
@@ -392,21 +411,20 @@ __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int 
     const R a = AX(i, j, k);
     R v;
     if (STD) {
-      const R y1 = (fabs(XX(i - 1, j + 1, k)) + fabs(XX(i, j + 1, k))) -
-                   (fabs(XX(i - 1, j - 1, k)) + fabs(XX(i, j - 1, k)));
-      const R y2 = fabs(XX(i - 1, j + 1, k)) + fabs(XX(i, j + 1, k)) + fabs(XX(i - 1, j - 1, k)) +
-                   fabs(XX(i, j - 1, k)) + ep;
+      const R p = PS ? P.cp.ld(i, QY(j + 1), k) : fabs(XX(i - 1, j + 1, k)) + fabs(XX(i, j + 1, k));
+      const R m0 = fabs(XX(i - 1, j - 1, k)), m1 = fabs(XX(i, j - 1, k));
+      const R y1 = STD_Y1(p, P.cp.ld(i, QY(j - 1), k), m0, m1), y2 = STD_Y2(p, m0, m1);
       if (GV)
         v = vdyfa_k(XX(i - 1, j, k), XX(i, j, k), P.gvs[0].ld(i, j, k), ep) +
             vcorra_b<U>(P.gvs[1].ld(i, j, k), y1, y2, hmx);
       else
-        v = vdyfa_u<U>(XX(i - 1, j, k), XX(i, j, k), a, hmx, ep) +
+        v = (PS ? vdyfa_s<U>(XX(i - 1, j, k), XX(i, j, k), a, hmx, P.cp.ld(i, j, k), ep)
+                : vdyfa_u<U>(XX(i - 1, j, k), XX(i, j, k), a, hmx, ep)) +
             vcorra_u<U>(a, S2X, y1, y2, hmx);
       if (zt) {
-        const R z1 = (fabs(XX(i - 1, j, k + 1)) + fabs(XX(i, j, k + 1))) -
-                     (fabs(XX(i - 1, j, k - 1)) + fabs(XX(i, j, k - 1)));
-        const R z2 = fabs(XX(i - 1, j, k + 1)) + fabs(XX(i, j, k + 1)) + fabs(XX(i - 1, j, k - 1)) +
-                     fabs(XX(i, j, k - 1)) + ep;
+        const R q = PS ? P.cp.ld(i, j, MZ(k + 1)) : fabs(XX(i - 1, j, k + 1)) + fabs(XX(i, j, k + 1));
+        const R n0 = fabs(XX(i - 1, j, k - 1)), n1 = fabs(XX(i, j, k - 1));
+        const R z1 = STD_Y1(q, P.cp.ld(i, j, MZ(k - 1)), n0, n1), z2 = STD_Y2(q, n0, n1);
         v = v + (GV ? vcorra_b<U>(P.gvs[2].ld(i, j, k), z1, z2, hmx)
                     : vcorra_u<U>(a, S3X, z1, z2,
                                   hmx));
@@ -434,21 +452,20 @@ __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int 
     const R a = AY(i, j, k);
     R v;
     if (STD) {
-      const R y1 = (fabs(XX(i + 1, j - 1, k)) + fabs(XX(i + 1, j, k))) -
-                   (fabs(XX(i - 1, j - 1, k)) + fabs(XX(i - 1, j, k)));
-      const R y2 = fabs(XX(i + 1, j - 1, k)) + fabs(XX(i + 1, j, k)) + fabs(XX(i - 1, j - 1, k)) +
-                   fabs(XX(i - 1, j, k)) + ep;
+      const R p = PS ? P.cn.ld(QX(i + 1), j, k) : fabs(XX(i + 1, j - 1, k)) + fabs(XX(i + 1, j, k));
+      const R m0 = fabs(XX(i - 1, j - 1, k)), m1 = fabs(XX(i - 1, j, k));
+      const R y1 = STD_Y1(p, P.cn.ld(QX(i - 1), j, k), m0, m1), y2 = STD_Y2(p, m0, m1);
       if (GV)
         v = vdyfa_k(XX(i, j - 1, k), XX(i, j, k), P.gvs[3].ld(i, j, k), ep) +
             vcorra_b<U>(P.gvs[4].ld(i, j, k), y1, y2, hmy);
       else
-        v = vdyfa_u<U>(XX(i, j - 1, k), XX(i, j, k), a, hmy, ep) +
+        v = (PS ? vdyfa_s<U>(XX(i, j - 1, k), XX(i, j, k), a, hmy, P.cn.ld(i, j, k), ep)
+                : vdyfa_u<U>(XX(i, j - 1, k), XX(i, j, k), a, hmy, ep)) +
             vcorra_u<U>(a, S1Y, y1, y2, hmy);
       if (zt) {
-        const R z1 = (fabs(XX(i, j - 1, k + 1)) + fabs(XX(i, j, k + 1))) -
-                     (fabs(XX(i, j - 1, k - 1)) + fabs(XX(i, j, k - 1)));
-        const R z2 = fabs(XX(i, j - 1, k + 1)) + fabs(XX(i, j, k + 1)) + fabs(XX(i, j - 1, k - 1)) +
-                     fabs(XX(i, j, k - 1)) + ep;
+        const R q = PS ? P.cn.ld(i, j, MZ(k + 1)) : fabs(XX(i, j - 1, k + 1)) + fabs(XX(i, j, k + 1));
+        const R n0 = fabs(XX(i, j - 1, k - 1)), n1 = fabs(XX(i, j, k - 1));
+        const R z1 = STD_Y1(q, P.cn.ld(i, j, MZ(k - 1)), n0, n1), z2 = STD_Y2(q, n0, n1);
         v = v + (GV ? vcorra_b<U>(P.gvs[5].ld(i, j, k), z1, z2, hmy)
                     : vcorra_u<U>(a, S3Y, z1, z2,
                                   hmy));
@@ -476,19 +493,18 @@ __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int 
     const R a = AZ(i, j, k);
     R v;
     if (STD) {
-      const R x1 = (fabs(XX(i + 1, j, k - 1)) + fabs(XX(i + 1, j, k))) -
-                   (fabs(XX(i - 1, j, k - 1)) + fabs(XX(i - 1, j, k)));
-      const R x2 = fabs(XX(i + 1, j, k - 1)) + fabs(XX(i + 1, j, k)) + fabs(XX(i - 1, j, k - 1)) +
-                   fabs(XX(i - 1, j, k)) + ep;
-      const R y1 = (fabs(XX(i, j + 1, k - 1)) + fabs(XX(i, j + 1, k))) -
-                   (fabs(XX(i, j - 1, k - 1)) + fabs(XX(i, j - 1, k)));
-      const R y2 = fabs(XX(i, j + 1, k - 1)) + fabs(XX(i, j + 1, k)) + fabs(XX(i, j - 1, k - 1)) +
-                   fabs(XX(i, j - 1, k)) + ep;
+      const R p = PS ? P.q.ld(QX(i + 1), j, k) : fabs(XX(i + 1, j, k - 1)) + fabs(XX(i + 1, j, k));
+      const R m0 = fabs(XX(i - 1, j, k - 1)), m1 = fabs(XX(i - 1, j, k));
+      const R x1 = STD_Y1(p, P.q.ld(QX(i - 1), j, k), m0, m1), x2 = STD_Y2(p, m0, m1);
+      const R q = PS ? P.q.ld(i, QY(j + 1), k) : fabs(XX(i, j + 1, k - 1)) + fabs(XX(i, j + 1, k));
+      const R n0 = fabs(XX(i, j - 1, k - 1)), n1 = fabs(XX(i, j - 1, k));
+      const R y1 = STD_Y1(q, P.q.ld(i, QY(j - 1), k), n0, n1), y2 = STD_Y2(q, n0, n1);
       if (GV)
         v = vdyfa_k(XX(i, j, k - 1), XX(i, j, k), P.gvs[6].ld(i, j, k), ep) +
             vcorra_b<U>(P.gvs[7].ld(i, j, k), x1, x2, hmz) + vcorra_b<U>(P.gvs[8].ld(i, j, k), y1, y2, hmz);
       else
-        v = vdyfa_u<U>(XX(i, j, k - 1), XX(i, j, k), a, hmz, ep) +
+        v = (PS ? vdyfa_s<U>(XX(i, j, k - 1), XX(i, j, k), a, hmz, P.q.ld(i, j, k), ep)
+                : vdyfa_u<U>(XX(i, j, k - 1), XX(i, j, k), a, hmz, ep)) +
             vcorra_u<U>(a, S1Z, x1, x2, hmz) +
             vcorra_u<U>(a, S2Z, y1, y2, hmz);
       put(2, v, donor(XX(i, j, k - 1), XX(i, j, k), v));
@@ -531,6 +547,8 @@ __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int 
 #undef S3Y
 #undef S1Z
 #undef S2Z
+#undef STD_Y1
+#undef STD_Y2
 #undef XX
 #undef AX
 #undef AY
@@ -541,7 +559,7 @@ template <class R, bool AIN, bool IN = false, bool U = false, bool PS = false, b
           bool PV = false>
 __device__ __forceinline__ void pseudo_body(const Prob<R>& P, int i, int j, int k) {
   if (P.stdf)
-    pseudo_form<R, true, AIN, IN, U, false, GV, DEFER>(P, i, j, k);
+    pseudo_form<R, true, AIN, IN, U, PS && !GV, GV, DEFER, PV>(P, i, j, k);
   else
     pseudo_form<R, false, AIN, IN, U, PS, GV, DEFER, PV>(P, i, j, k);
 }
@@ -783,11 +801,15 @@ __device__ __forceinline__ void block_ratios(const Prob<R>& P, int i, int j, int
 // into f1, a2(j)+a2(j+1) into f2, a3(k)+a3(k+1) into f3, which the gauge form
 // leaves unused outside the density step.  The face reads take the boundary
 // rules, so the pairs interior warps read are the sums their faces give.
-template <class R, bool AIN = true, bool PV = false>
+// STD: the standard form's pairs are sums of magnitudes, |x(i-1)|+|x(i)| and so on
+// (antidiff3d-standard-gpubc.f90:72-203), and its velocity pairs, in the first
+// pass alone, go to w1..w3.
+template <class R, bool AIN = true, bool PV = false, bool STD = false>
 __device__ __forceinline__ void pairs_body(const Prob<R>& P, int i, int j, int k) {
   const Geo& g = P.g;
   const Arr<R>& X = P.xant;
-  const R x = X.ld(i, j, k);
+  auto val = [&](int a, int b, int c) { return STD ? fabs(X.ld(a, b, c)) : X.ld(a, b, c); };
+  const R x = val(i, j, k);
   R a1 = R(0), a2 = R(0), a3 = R(0);
   if (PV) {
     const Arr<R>& A1 = AIN ? P.u1 : P.w1;
@@ -797,13 +819,13 @@ __device__ __forceinline__ void pairs_body(const Prob<R>& P, int i, int j, int k
     a2 = fy<R, AIN>(g, A2, i, j, k) + fy<R, AIN>(g, A2, i, j + 1, k);
     a3 = fz<R, AIN>(g, A3, i, j, k) + fz<R, AIN>(g, A3, i, j, k + 1);
   }
-  if (i > 1 || g.bx) P.cp.at(i, j, k) = x + X.ld(i > 1 ? i - 1 : g.np, j, k);
-  if (j > 1 || g.by) P.cn.at(i, j, k) = x + X.ld(i, j > 1 ? j - 1 : g.mp, k);
-  if (k > 1 || g.bz) P.q.at(i, j, k) = x + X.ld(i, j, k > 1 ? k - 1 : g.lp);
+  if (i > 1 || g.bx) P.cp.at(i, j, k) = x + val(i > 1 ? i - 1 : g.np, j, k);
+  if (j > 1 || g.by) P.cn.at(i, j, k) = x + val(i, j > 1 ? j - 1 : g.mp, k);
+  if (k > 1 || g.bz) P.q.at(i, j, k) = x + val(i, j, k > 1 ? k - 1 : g.lp);
   if (PV) {
-    P.f1.at(i, j, k) = a1;
-    P.f2.at(i, j, k) = a2;
-    P.f3.at(i, j, k) = a3;
+    (STD ? P.w1 : P.f1).at(i, j, k) = a1;
+    (STD ? P.w2 : P.f2).at(i, j, k) = a2;
+    (STD ? P.w3 : P.f3).at(i, j, k) = a3;
   }
 }
 

@@ -337,6 +337,10 @@ template <bool U, class R> __device__ __forceinline__ R vdyf_u(R x1, R x2, R a, 
 template <bool U, class R> __device__ __forceinline__ R vdyfa_u(R x1, R x2, R a, R hm, R ep) {
   return quot((fabs(a) - hmul<U>(a * a, hm)) * (fabs(x2) - fabs(x1)), fabs(x2) + fabs(x1) + ep);
 }
+// vdyfa_u with |x1|+|x2| at hand (sum)
+template <bool U, class R> __device__ __forceinline__ R vdyfa_s(R x1, R x2, R a, R hm, R sum, R ep) {
+  return quot((fabs(a) - hmul<U>(a * a, hm)) * (fabs(x2) - fabs(x1)), sum + ep);
+}
 template <bool U, class R> __device__ __forceinline__ R vcorra_u(R a, R b, R y1, R y2, R hm) {
   return -quot(hmul<U>(scale_down<3>(a) * b * y1, hm), y2);
 }

@@ -128,50 +128,44 @@ __global__ void __launch_bounds__(128, PseudoMinBlocks<R>::v) k_pseudo(const Pro
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
   const bool win = warp_interior(P.g, i, j, k);
-  // FP64 with every pair sum stored: full warps at a boundary read them too,
-  // through the boundary maps
-  bool pin = false;
-  if constexpr (sizeof(R) == 8)
-    if (!win && P.pairs == 2) pin = warp_on_grid(P.g, i, j);
-  if (i > P.g.np || j > P.g.mp) return;
-  if (!win) {
-    if constexpr (sizeof(R) == 8) {
-      if (pin) {
-        if (warp_unit_faces(P, i, j, k))
-          pseudo_body<R, AIN, false, true, true, false, D, true>(P, i, j, k);
+  const bool valid = i <= P.g.np && j <= P.g.mp;
+  const unsigned act = __ballot_sync(0xffffffffu, valid);
+  if (!valid) return;
+  if constexpr (sizeof(R) == 8) {
+    // every warp reads the stored pair sums, those at a boundary through the
+    // boundary maps; the velocity pairs too where they are stored (pairs 2)
+    const bool unit = warp_unit_faces(P, i, j, k, act);
+    if (win) {
+      if (P.pairs == 2) {
+        if (unit)
+          pseudo_body<R, AIN, true, true, true, false, D, true>(P, i, j, k);
         else
-          pseudo_body<R, AIN, false, false, true, false, D, true>(P, i, j, k);
-        return;
+          pseudo_body<R, AIN, true, false, true, false, D, true>(P, i, j, k);
+      } else {
+        if (unit)
+          pseudo_body<R, AIN, true, true, true, false, D>(P, i, j, k);
+        else
+          pseudo_body<R, AIN, true, false, true, false, D>(P, i, j, k);
       }
-    }
-    pseudo_body<R, AIN, false, false, false, false, D>(P, i, j, k);
-  } else if constexpr (sizeof(R) == 8) {
-    const bool unit = warp_unit_faces(P, i, j, k);
-    if (P.pairs == 2) {
+    } else if (P.pairs == 2) {
       if (unit)
-        pseudo_body<R, AIN, true, true, true, false, D, true>(P, i, j, k);
+        pseudo_body<R, AIN, false, true, true, false, D, true>(P, i, j, k);
       else
-        pseudo_body<R, AIN, true, false, true, false, D, true>(P, i, j, k);
-    } else if (P.pairs) {
-      if (unit)
-        pseudo_body<R, AIN, true, true, true, false, D>(P, i, j, k);
-      else
-        pseudo_body<R, AIN, true, false, true, false, D>(P, i, j, k);
+        pseudo_body<R, AIN, false, false, true, false, D, true>(P, i, j, k);
     } else {
-      if (unit)
-        pseudo_body<R, AIN, true, true, false, false, D>(P, i, j, k);
-      else
-        pseudo_body<R, AIN, true, false, false, false, D>(P, i, j, k);
+      pseudo_body<R, AIN, false, false, true, false, D>(P, i, j, k);
     }
-  } else {
+  } else if (win) {
     pseudo_body<R, AIN, true, false, false, false, D>(P, i, j, k);
+  } else {
+    pseudo_body<R, AIN, false, false, false, false, D>(P, i, j, k);
   }
 }
 
-template <class R, bool AIN, bool PV>
+template <class R, bool AIN, bool PV, bool STD>
 __global__ void __launch_bounds__(128) k_pairs(const Prob<R> P) {
   CELL_INDEX
-  pairs_body<R, AIN, PV>(P, i, j, k);
+  pairs_body<R, AIN, PV, STD>(P, i, j, k);
 }
 template <class R, bool NONOS, bool FIRST, bool KEEP>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_BOUNDS_F64, MPDATA_MINB_BOUNDS_F32>::v)) k_bounds(const Prob<R> P) {
@@ -243,16 +237,22 @@ int run_step(const Prob<R>& P, int iord, int nonos, Prof* prof, cudaStream_t s) 
   }
   LAUNCH(ST_UPWIND, (k_upwind<R, true><<<grd, blk, 0, s>>>(P)));
   const bool keep = iord > 2;
-  // FP64 gauge form: the pseudo-velocity stage reads precomputed pair sums of
-  // xant (pairs 1) and, outside the density step, whose upwind fluxes hold
-  // f1..f3, of the pass velocities too (pairs 2)
+  // FP64: the pseudo-velocity stage reads precomputed pair sums of xant (pairs 1)
+  // and, where three fields are free for them, of the pass velocities too (pairs
+  // 2): not in the density step, whose upwind fluxes hold f1..f3, and in the
+  // standard form in the first pass alone, whose w1..w3 are not yet written.  The
+  // standard form went from 102 to 75 FP64 additions and products per cell and pass.
   Prob<R> Q = P;
-  Q.pairs = (!P.stdf && sizeof(R) == 8) ? (P.rho ? 1 : 2) : 0;
   for (int pass = 2; pass <= iord; pass++) {
     const bool first = (pass == 2), last = (pass == iord);
-    if (Q.pairs == 2 && first) LAUNCH(ST_PAIRS, (k_pairs<R, true, true><<<grd, blk, 0, s>>>(Q)));
-    else if (Q.pairs == 2) LAUNCH(ST_PAIRS, (k_pairs<R, false, true><<<grd, blk, 0, s>>>(Q)));
-    else if (Q.pairs) LAUNCH(ST_PAIRS, (k_pairs<R, true, false><<<grd, blk, 0, s>>>(Q)));
+    if constexpr (sizeof(R) == 8) {
+      Q.pairs = P.rho || (P.stdf && !first) ? 1 : 2;
+      if (P.stdf && first) LAUNCH(ST_PAIRS, (k_pairs<R, true, true, true><<<grd, blk, 0, s>>>(Q)));
+      else if (P.stdf) LAUNCH(ST_PAIRS, (k_pairs<R, false, false, true><<<grd, blk, 0, s>>>(Q)));
+      else if (P.rho) LAUNCH(ST_PAIRS, (k_pairs<R, true, false, false><<<grd, blk, 0, s>>>(Q)));
+      else if (first) LAUNCH(ST_PAIRS, (k_pairs<R, true, true, false><<<grd, blk, 0, s>>>(Q)));
+      else LAUNCH(ST_PAIRS, (k_pairs<R, false, true, false><<<grd, blk, 0, s>>>(Q)));
+    }
     if (first) LAUNCH(ST_PSEUDO, (k_pseudo<R, true><<<grd, blk, 0, s>>>(Q)));
     else LAUNCH(ST_PSEUDO, (k_pseudo<R, false><<<grd, blk, 0, s>>>(Q)));
     if (!nonos) LAUNCH(ST_BOUNDS, (k_bounds<R, false, true, false><<<grd, blk, 0, s>>>(P)));
