@@ -22,11 +22,15 @@
 //                                                     the previous pass's lambda_w
 //   upwind    xant(psi, u)                         -> lambda_psi, lambda_u
 // Each reverse kernel walks the forward stage's reads (with the same boundary
-// index maps) and scatters the products of the local partial derivatives
-// with atomic adds, so wall faces (constant zero), mirrored z faces and
-// periodic wraps are transposed exactly as the forward reads them.  The
+// index maps), so wall faces (constant zero), mirrored z faces and periodic
+// wraps are transposed exactly as the forward reads them.  What belongs to the
+// cell or to a face it owns is stored; the rest is scattered with atomic adds
+// (the bounds, the pseudo-velocity in FP64 and at walls) or gathered.  The
 // summation order of the atomics is not fixed: results agree with the FP64
 // AD oracle to rounding, not bit for bit.
+// Gauge form, per field of 256x256x64 FP64 cells (33 MB): clearing all 19
+// accumulators took 95 us of a step adjoint; only those that the first kernel
+// to touch them adds to are cleared now (lcp and lcn at iord 2).
 #include "mpdata_body.cuh"
 #include "mpdata_stages.cuh"
 
@@ -142,6 +146,10 @@ template <class R> __device__ __forceinline__ R dpn(R y) { return (sgn(y) && non
 template <class R> __device__ __forceinline__ R dabs(R y) { return sgn(y) ? R(-1) : R(1); }
 
 
+template <class R> __device__ __forceinline__ R negv(R x) { return -x; }
+template <> __device__ __forceinline__ double negv<double>(double x) { return neg_bits(x); }
+__device__ __forceinline__ bool is_one(float v) { return v == 1.0f; }
+
 // Reverse kernels: the body is a device function of (i,j,k) templated on
 // IN; warps away from every wall take IN = true.
 #define ADISPATCH(CALL)                                      \
@@ -164,26 +172,30 @@ template <class R> __device__ __forceinline__ R dabs(R y) { return sgn(y) ? R(-1
   const Geo& g = P.g;
 
 // ---- update: x_new = rhr*(q - D/h), D = sum of signed limited fluxes -------
-template <class R, bool IN>
-__device__ __forceinline__ void ka_update_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
-  const Geo& g = P.g;
-  const R ln = A.lam.ld(i, j, k);
-  const R rh = P.rhr.ld(i, j, k);
-  const R lt = rh * ln;                 // d x_new / d t, t = q - D/h
-  A.lxant.at(i, j, k) = quot(lt, rh);        // q = xant/rhr
-  const R lD = quot(-lt, P.h.ld(i, j, k));
-  fx_add<R, false, IN>(g, A.lw1, i + 1, j, k, lD);
-  fx_add<R, false, IN>(g, A.lw1, i, j, k, -lD);
-  fy_add<R, false, IN>(g, A.lw2, i, j + 1, k, lD);
-  fy_add<R, false, IN>(g, A.lw2, i, j, k, -lD);
-  fz_add<R, false, IN>(g, A.lw3, i, j, k + 1, lD);
-  fz_add<R, false, IN>(g, A.lw3, i, j, k, -lD);
-}
+// The adjoint of D is one value per cell (lq); the limiter's reverse takes a
+// face's lambda_w from the two cells it separates, so nothing is scattered.
+// After the last pass's read of the caller's lambda (A.lx set), that array
+// becomes the accumulator of the step input's adjoint.  256x256x64 FP64: 31 us,
+// at the rate of its five fields; six atomics a cell took 61.
 template <class R>
 __global__ void KA_LB_UPDATE ka_update(const Prob<R> P, const AdjArr<R> A) {
-#define C(IN) ka_update_cell<R, IN>(P, A, i, j, k)
-  ADISPATCH(C)
-#undef C
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int k = blockIdx.z + 1;
+  const bool in = i <= P.g.np && j <= P.g.mp;
+  const unsigned act = __ballot_sync(0xffffffffu, in);
+  if (!in) return;
+  const R ln = A.lam.ld(i, j, k);
+  const R rh = P.rhr.ld(i, j, k), h = P.h.ld(i, j, k);
+  if (A.lx.p) A.lx.at(i, j, k) = R(0);
+  if (__all_sync(act, is_one(rh) && is_one(h))) {  // x*1 == x/1 == x
+    A.lxant.at(i, j, k) = ln;
+    A.lq.at(i, j, k) = negv(ln);
+    return;
+  }
+  const R lt = rh * ln;                 // d x_new / d t, t = q - D/h
+  A.lxant.at(i, j, k) = quot(lt, rh);   // q = xant/rhr
+  A.lq.at(i, j, k) = quot(-lt, h);
 }
 
 // ---- limiter: w = pp(v)*min3(cp(c),cn(c-1)) - pn(v)*min3(cp(c-1),cn(c)) -------
@@ -194,39 +206,63 @@ __device__ __forceinline__ bool lt_nonneg(double a, double b) {
   return __double_as_longlong(a) < __double_as_longlong(b);
 }
 __device__ __forceinline__ bool lt_nonneg(float a, float b) { return a < b; }
+template <class R> __device__ __forceinline__ bool min3_takes_b(R a, R b) {
+  return !lt_nonneg(lt_nonneg(R(1), a) ? R(1) : a, b);
+}
+template <class R> __device__ __forceinline__ bool min3_takes_a(R a, R b) {
+  return !min3_takes_b(a, b) && !lt_nonneg(R(1), a);
+}
 template <class R>
 __device__ __forceinline__ void min3_adj(R a, R b, R lam, const Arr<R>& La, int ia, int ja, int ka,
                                          const Arr<R>& Lb, int ib, int jb, int kb) {
-  const bool a_over = lt_nonneg(R(1), a);
-  const R t = a_over ? R(1) : a;
-  if (!lt_nonneg(t, b)) { addat(Lb, ib, jb, kb, lam); return; }
-  if (!a_over) addat(La, ia, ja, ka, lam);
+  if (min3_takes_b(a, b)) addat(Lb, ib, jb, kb, lam);
+  else if (min3_takes_a(a, b)) addat(La, ia, ja, ka, lam);
 }
 
+// A cell owns its lower face on each axis.  The face's lambda_w is lq of the
+// cell below minus lq of the cell above; at a z wall the mirrored face doubles
+// the wall cell's share of its inner face (exact).  LW, where it is given,
+// holds what the next pass (or the density step's mass fluxes) added to
+// lambda_w.  lambda_v is stored whole (the bounds' reverse adds to it); only
+// the ratios that limit their flux, a minority, are added to by atomics.
 template <class R, bool NONOS, bool IN>
 __device__ __forceinline__ void ka_limit_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
   const Geo& g = P.g;
   const R cpc = NONOS ? P.cp.ld(i, j, k) : R(0), cnc = NONOS ? P.cn.ld(i, j, k) : R(0);
-#define LIMIT_FACE(V, LV, LW, IM, JM, KM)                                                  \
+  const R lqc = A.lq.ld(i, j, k);
+#define LIMIT_FACE(V, LV, LW, IM, JM, KM, LQL, LQR)                                        \
   {                                                                                        \
     const R v = V.ld(i, j, k);                                                             \
-    const R lw = LW.ld(i, j, k);                                                           \
+    R lw = (LQL) - (LQR);                                                                  \
+    if (LW.p) lw += LW.ld(i, j, k);                                                        \
     if (!NONOS) {                                                                          \
-      addat(LV, i, j, k, lw);                                                              \
+      LV.at(i, j, k) = lw;                                                                 \
     } else {                                                                               \
       const R cpm = P.cp.ld(IM, JM, KM), cnm = P.cn.ld(IM, JM, KM);                        \
       /* dw/dv = a1 (v > 0), a2 (v < 0), 0; dw/da1 = pp(v), dw/da2 = -pn(v): */          \
       /* one of them is v, the other zero */                                              \
       const bool vz = !nonzero(v), vn = sgn(v);                                             \
-      const R m = lw * v;                                                                   \
-      if (!vz) addat(LV, i, j, k, lw * (vn ? min3(cpm, cnc) : min3(cpc, cnm)));             \
-      if (!vz && !vn) min3_adj(cpc, cnm, m, A.lcp, i, j, k, A.lcn, IM, JM, KM);             \
-      if (!vz && vn) min3_adj(cpm, cnc, m, A.lcp, IM, JM, KM, A.lcn, i, j, k);              \
-    }                                                                                      \
+      const R a = vn ? cpm : cpc, b = vn ? cnc : cnm;                                       \
+      LV.at(i, j, k) = vz ? R(0) : lw * min3(a, b);                                         \
+      const bool tb = min3_takes_b(a, b), ta = !tb && !lt_nonneg(R(1), a);                  \
+      if (!vz && (ta || tb)) {                                                              \
+        const R m = lw * v;                                                                 \
+        const bool lower = vn == ta; /* cp is the donor-side operand a, cn is b */          \
+        atomicAdd(ta ? (lower ? &A.lcp.at(IM, JM, KM) : &A.lcp.at(i, j, k))                 \
+                     : (lower ? &A.lcn.at(IM, JM, KM) : &A.lcn.at(i, j, k)),                \
+                  m);                                                                       \
+      }                                                                                     \
+    }                                                                                       \
   }
-  if (IN || g.bx || i > 1) LIMIT_FACE(P.v1, A.lv1, A.lw1, (IN ? i - 1 : wrapi(i - 1, g.np)), j, k)
-  if (IN || g.by || j > 1) LIMIT_FACE(P.v2, A.lv2, A.lw2, i, (IN ? j - 1 : wrapi(j - 1, g.mp)), k)
-  if (IN || g.bz || k > 1) LIMIT_FACE(P.v3, A.lv3, A.lw3, i, j, (IN ? k - 1 : wrapi(k - 1, g.lp)))
+  const int im = IN ? i - 1 : wrapi(i - 1, g.np), jm = IN ? j - 1 : wrapi(j - 1, g.mp), km = IN ? k - 1 : wrapi(k - 1, g.lp);
+  if (IN || g.bx || i > 1) LIMIT_FACE(P.v1, A.lv1, A.lw1, im, j, k, A.lq.ld(im, j, k), lqc)
+  if (IN || g.by || j > 1) LIMIT_FACE(P.v2, A.lv2, A.lw2, i, jm, k, A.lq.ld(i, jm, k), lqc)
+  if (IN || g.bz || k > 1) {
+    R ql = A.lq.ld(i, j, km), qr = lqc;
+    if (!g.bz && k == 2) ql = scale_up<1>(ql);
+    if (!g.bz && k == g.lp) qr = scale_up<1>(qr);
+    LIMIT_FACE(P.v3, A.lv3, A.lw3, i, j, km, ql, qr)
+  }
 #undef LIMIT_FACE
 }
 template <class R, bool NONOS>
@@ -240,7 +276,9 @@ __global__ void KA_LB_LIMIT ka_limit(const Prob<R> P, const AdjArr<R> A) {
 // The extrema are re-folded in the oracle's order (mx2/mn2 trees) with the
 // compare-and-select's own semantics (ties, +0 == -0 included, keep the
 // second operand), so each goes to the same operand: element ids 0..6 are
-// x_in, 7..13 xant.  FP64 values compare on the integer pipe (ieee_gt).
+// x_in, 7..13 xant (centre 1 and 8; the lower and upper neighbours along x, y,
+// z at 0, 2, 3, 4, 5, 6 and 7 more).  FP64 values compare on the integer pipe
+// (ieee_gt).
 __device__ __forceinline__ bool arg_gt(double a, double b) { return ieee_gt(a, b); }
 __device__ __forceinline__ bool arg_gt(float a, float b) { return a > b; }
 template <class R>
@@ -251,6 +289,60 @@ struct Arg {
 template <class R> __device__ __forceinline__ Arg<R> mkarg(R v, int id) { return Arg<R>{v, id}; }
 template <class R> __device__ __forceinline__ Arg<R> amax(Arg<R> a, Arg<R> b) { return arg_gt(a.v, b.v) ? a : b; }
 template <class R> __device__ __forceinline__ Arg<R> amin(Arg<R> a, Arg<R> b) { return arg_gt(b.v, a.v) ? a : b; }
+
+// FIRST: the fold starts from the step input's star (ids 0..6); later passes
+// start from the previous pass's running extrema (id 14).  The current
+// field's star is ids 7..13.  x_in is read with the zero-gradient map, the
+// current field with the reflection map.
+template <class R, bool FIRST, bool IN>
+struct StarFold {
+  int im, ip, jm, jp, km, kp, ri_m, ri_p, rj_m, rj_p;
+  Arg<R> ma, mi;
+  __device__ __forceinline__ StarFold(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
+    const Geo& g = P.g;
+    const bool lo = IN || g.bz || k > 1, hi = IN || g.bz || k < g.lp;
+    im = IN ? i - 1 : (g.bx ? wrapi(i - 1, g.np) : clampi(i - 1, g.np));
+    ip = IN ? i + 1 : (g.bx ? wrapi(i + 1, g.np) : clampi(i + 1, g.np));
+    jm = IN ? j - 1 : (g.by ? wrapi(j - 1, g.mp) : clampi(j - 1, g.mp));
+    jp = IN ? j + 1 : (g.by ? wrapi(j + 1, g.mp) : clampi(j + 1, g.mp));
+    km = cz<IN>(g, k - 1);
+    kp = cz<IN>(g, k + 1);
+    ri_m = IN ? i - 1 : (g.bx ? wrapi(i - 1, g.np) : refl(i - 1, g.np));
+    ri_p = IN ? i + 1 : (g.bx ? wrapi(i + 1, g.np) : refl(i + 1, g.np));
+    rj_m = IN ? j - 1 : (g.by ? wrapi(j - 1, g.mp) : refl(j - 1, g.mp));
+    rj_p = IN ? j + 1 : (g.by ? wrapi(j + 1, g.mp) : refl(j + 1, g.mp));
+    const Arr<R>& X = P.xant;
+    const Arr<R>& xin = P.psi;
+    if (FIRST) {
+      const Arg<R> e0 = mkarg(xin.ld(im, j, k), 0), e1 = mkarg(xin.ld(i, j, k), 1), e2 = mkarg(xin.ld(ip, j, k), 2),
+                   e3 = mkarg(xin.ld(i, jm, k), 3), e4 = mkarg(xin.ld(i, jp, k), 4),
+                   e5 = mkarg(xin.ld(i, j, km), 5), e6 = mkarg(xin.ld(i, j, kp), 6);
+      ma = amax(amax(amax(e0, e1), amax(e2, e3)), e4);
+      mi = amin(amin(amin(e0, e1), amin(e2, e3)), e4);
+      if (lo) { ma = amax(ma, e5); mi = amin(mi, e5); }
+      if (hi) { ma = amax(ma, e6); mi = amin(mi, e6); }
+    } else {
+      ma = mkarg(A.mxp.ld(i, j, k), 14);
+      mi = mkarg(A.mnp.ld(i, j, k), 14);
+    }
+    const Arg<R> f0 = mkarg(X.ld(ri_m, j, k), 7), f1 = mkarg(X.ld(i, j, k), 8), f2 = mkarg(X.ld(ri_p, j, k), 9),
+                 f3 = mkarg(X.ld(i, rj_m, k), 10), f4 = mkarg(X.ld(i, rj_p, k), 11),
+                 f5 = mkarg(X.ld(i, j, km), 12), f6 = mkarg(X.ld(i, j, kp), 13);
+    ma = amax(amax(amax(ma, f0), amax(f1, f2)), amax(f3, f4));
+    mi = amin(amin(amin(mi, f0), amin(f1, f2)), amin(f3, f4));
+    if (lo) { ma = amax(ma, f5); mi = amin(mi, f5); }
+    if (hi) { ma = amax(ma, f6); mi = amin(mi, f6); }
+  }
+  // adds v to the adjoint of the element id (not 14)
+  __device__ __forceinline__ void add(const AdjArr<R>& A, int id, int i, int j, int k, R v) const {
+    const bool in = FIRST && id < 7;
+    const int n = in ? id : id - 7;
+    const int ii = n == 0 ? (in ? im : ri_m) : n == 2 ? (in ? ip : ri_p) : i;
+    const int jj = n == 3 ? (in ? jm : rj_m) : n == 4 ? (in ? jp : rj_p) : j;
+    const int kk = n == 5 ? km : n == 6 ? kp : k;
+    addat(in ? A.lx : A.lxant, ii, jj, kk, v);
+  }
+};
 
 // Adjoint of the bounds' denominators onto one flux f: Dp holds pn(f) and
 // Dn pp(f) for an outflow face (e), the reverse for an inflow face (w); a
@@ -263,50 +355,12 @@ __device__ __forceinline__ R lflux(R f, R lDp, R lDn, bool inflow) {
   return neg ? -lDp : lDn;
 }
 
-// FIRST: the fold starts from the step input's star (ids 0..6); later passes
-// start from the previous pass's running extrema (id 14).  The current
-// field's star is ids 7..13.  The adjoint of this pass's extrema is the
-// cp/cn part plus what the next pass carried back (lmx, lmn).
 // STD: the fluxes of the bounds are the unlimited donor fluxes f*ns (their
 // adjoint goes to lf); gauge: the pseudo-velocities themselves (lv).
 template <class R, bool FIRST, bool STD, bool IN>
 __device__ __forceinline__ void ka_bounds_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
   const Geo& g = P.g;
-  const bool lo = IN || g.bz || k > 1, hi = IN || g.bz || k < g.lp;
-  const Arr<R>& X = P.xant;
-  const Arr<R>& xin = P.psi;
-  // star cells: x_in with the zero-gradient map, the current field with the reflection map
-  const int im = IN ? i - 1 : (g.bx ? wrapi(i - 1, g.np) : clampi(i - 1, g.np));
-  const int ip = IN ? i + 1 : (g.bx ? wrapi(i + 1, g.np) : clampi(i + 1, g.np));
-  const int jm = IN ? j - 1 : (g.by ? wrapi(j - 1, g.mp) : clampi(j - 1, g.mp));
-  const int jp = IN ? j + 1 : (g.by ? wrapi(j + 1, g.mp) : clampi(j + 1, g.mp));
-  const int km = cz<IN>(g, k - 1), kp = cz<IN>(g, k + 1);
-  const int ri_m = IN ? i - 1 : (g.bx ? wrapi(i - 1, g.np) : refl(i - 1, g.np)), ri_p = IN ? i + 1 : (g.bx ? wrapi(i + 1, g.np) : refl(i + 1, g.np));
-  const int rj_m = IN ? j - 1 : (g.by ? wrapi(j - 1, g.mp) : refl(j - 1, g.mp)), rj_p = IN ? j + 1 : (g.by ? wrapi(j + 1, g.mp) : refl(j + 1, g.mp));
-  // element table: (i,j,k) of ids 0..13; id 14 is the previous extremum at (i,j,k)
-  const int ci[15] = {im, i, ip, i, i, i, i, ri_m, i, ri_p, i, i, i, i, i};
-  const int cj[15] = {j, j, j, jm, jp, j, j, j, j, j, rj_m, rj_p, j, j, j};
-  const int ck[15] = {k, k, k, k, k, km, kp, k, k, k, k, k, km, kp, k};
-  Arg<R> e[14];
-  for (int n = 7; n < 14; n++) e[n] = mkarg(X.ld(ci[n], cj[n], ck[n]), n);
-  Arg<R> ma, mi;
-  if (FIRST) {
-    for (int n = 0; n < 7; n++) e[n] = mkarg(xin.ld(ci[n], cj[n], ck[n]), n);
-    ma = amax(amax(amax(e[0], e[1]), amax(e[2], e[3])), e[4]);
-    mi = amin(amin(amin(e[0], e[1]), amin(e[2], e[3])), e[4]);
-    if (lo) { ma = amax(ma, e[5]); mi = amin(mi, e[5]); }
-    if (hi) { ma = amax(ma, e[6]); mi = amin(mi, e[6]); }
-  } else {
-    ma = mkarg(A.mxp.ld(i, j, k), 14);
-    mi = mkarg(A.mnp.ld(i, j, k), 14);
-  }
-  ma = amax(amax(amax(ma, e[7]), amax(e[8], e[9])), amax(e[10], e[11]));
-  mi = amin(amin(amin(mi, e[7]), amin(e[8], e[9])), amin(e[10], e[11]));
-  if (lo) { ma = amax(ma, e[12]); mi = amin(mi, e[12]); }
-  if (hi) { ma = amax(ma, e[13]); mi = amin(mi, e[13]); }
-
-  const R x = X.ld(i, j, k), hc = P.h.ld(i, j, k);
-  const R lcp = A.lcp.ld(i, j, k), lcn = A.lcn.ld(i, j, k);
+  const StarFold<R, FIRST, IN> x(P, A, i, j, k);
   const Arr<R>& F1 = STD ? P.f1 : P.v1;
   const Arr<R>& F2 = STD ? P.f2 : P.v2;
   const Arr<R>& F3 = STD ? P.f3 : P.v3;
@@ -316,26 +370,29 @@ __device__ __forceinline__ void ka_bounds_cell(const Prob<R>& P, const AdjArr<R>
   const R e1 = fx<R, false, IN>(g, F1, i + 1, j, k), w1 = fx<R, false, IN>(g, F1, i, j, k);
   const R e2 = fy<R, false, IN>(g, F2, i, j + 1, k), w2 = fy<R, false, IN>(g, F2, i, j, k);
   const R e3 = fz<R, false, IN>(g, F3, i, j, k + 1), w3 = fz<R, false, IN>(g, F3, i, j, k);
-  // d cp/d mx, d cn/d mn (plus the carried adjoints of the extrema), d/d x,
-  // and d/dD = -c/D.  cp = num/Dp: lnum = lcp*h/Dp, lDp = -lnum*(mx-x)/Dp,
-  // with one reciprocal per denominator; both vanish where the limiter did
-  // not select the ratio (lcp = 0), as they mostly do.
+  // d cp/d mx, d cn/d mn, d/d x, and d/dD = -c/D.  cp = num/Dp: lnum =
+  // lcp*h/Dp, lDp = -lnum*(mx-x)/Dp, with one reciprocal per denominator.
+  const R lcp = A.lcp.ld(i, j, k), lcn = A.lcn.ld(i, j, k);
   R lnum_p = R(0), lnum_n = R(0), lDp = R(0), lDn = R(0);
   if (nonzero(lcp) || nonzero(lcn)) {
+    const R xc = P.xant.ld(i, j, k), hc = P.h.ld(i, j, k);
     const R ep = Eps<R>::v;
     const R Dp = pn(e1) + pp(w1) + pn(e2) + pp(w2) + pn(e3) + pp(w3) + ep;
     const R Dn = pp(e1) + pn(w1) + pp(e2) + pn(w2) + pp(e3) + pn(w3) + ep;
     const R rp = quot(R(1), Dp), rn = quot(R(1), Dn);
     lnum_p = lcp * hc * rp;
     lnum_n = lcn * hc * rn;
-    lDp = -(lnum_p * (ma.v - x)) * rp;
-    lDn = -(lnum_n * (x - mi.v)) * rn;
+    lDp = -(lnum_p * (x.ma.v - xc)) * rp;
+    lDn = -(lnum_n * (xc - x.mi.v)) * rn;
   }
-  const R lma = lnum_p + A.lmx.ld(i, j, k), lmi = -lnum_n + A.lmn.ld(i, j, k);
-  if (ma.id == 14) addat(A.lmxp, i, j, k, lma);
-  else addat(ma.id < 7 ? A.lx : A.lxant, ci[ma.id], cj[ma.id], ck[ma.id], lma);
-  if (mi.id == 14) addat(A.lmnp, i, j, k, lmi);
-  else addat(mi.id < 7 ? A.lx : A.lxant, ci[mi.id], cj[mi.id], ck[mi.id], lmi);
+  // the adjoint of this pass's extrema: the ratios' part and what the next
+  // pass carried back (lmx, lmn)
+  const R lma = A.lmx.p ? lnum_p + A.lmx.ld(i, j, k) : lnum_p;
+  const R lmi = A.lmn.p ? -lnum_n + A.lmn.ld(i, j, k) : -lnum_n;
+  if (!FIRST && x.ma.id == 14) addat(A.lmxp, i, j, k, lma);
+  else x.add(A, x.ma.id, i, j, k, lma);
+  if (!FIRST && x.mi.id == 14) addat(A.lmnp, i, j, k, lmi);
+  else x.add(A, x.mi.id, i, j, k, lmi);
   addat(A.lxant, i, j, k, lnum_n - lnum_p);
   // Dp = pn(e)+pp(w)+..., Dn = pp(e)+pn(w)+... over the six faces
   fx_add<R, false, IN>(g, LF1, i + 1, j, k, lflux(e1, lDp, lDn, false));
@@ -345,11 +402,39 @@ __device__ __forceinline__ void ka_bounds_cell(const Prob<R>& P, const AdjArr<R>
   fz_add<R, false, IN>(g, LF3, i, j, k + 1, lflux(e3, lDp, lDn, false));
   fz_add<R, false, IN>(g, LF3, i, j, k, lflux(w3, lDp, lDn, true));
 }
+// Only a cell whose ratios limit a flux, or whose extrema carry an adjoint
+// back, contributes; the rest (about nine in ten on a random field) need no
+// fold of 14 values and no quotient.  A warp's row holds a few such cells, so
+// the block of 128 packs its cells first and its leading warps take them.
+// 256x256x64 FP64: 190 us, 338 with every cell in its own lane; FP32
+// 128x128x64: 25 us, 37 before.
 template <class R, bool FIRST, bool STD>
 __global__ void KA_LB_BOUNDS ka_bounds(const Prob<R> P, const AdjArr<R> A) {
-#define C(IN) ka_bounds_cell<R, FIRST, STD, IN>(P, A, i, j, k)
-  ADISPATCH(C)
-#undef C
+  __shared__ int list[128];
+  __shared__ int count;
+  const Geo& g = P.g;
+  const int k = blockIdx.z + 1;
+  const int t = threadIdx.y * 32 + threadIdx.x;
+  int i = blockIdx.x * 32 + threadIdx.x + 1, j = blockIdx.y * 4 + threadIdx.y + 1;
+  if (t == 0) count = 0;
+  __syncthreads();
+  bool act = false;
+  if (i <= g.np && j <= g.mp) {
+    act = nonzero(A.lcp.ld(i, j, k)) || nonzero(A.lcn.ld(i, j, k));
+    if (A.lmx.p) act = act || nonzero(A.lmx.ld(i, j, k)) || nonzero(A.lmn.ld(i, j, k));
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, act);
+  int base = 0;
+  if (threadIdx.x == 0 && m) base = atomicAdd(&count, __popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (act) list[base + __popc(m & ((1u << threadIdx.x) - 1u))] = t;
+  __syncthreads();
+  if (t >= count) return;
+  const int c = list[t];
+  i = blockIdx.x * 32 + (c & 31) + 1;
+  j = blockIdx.y * 4 + (c >> 5) + 1;
+  if (i >= 2 && i < g.np && j >= 2 && j < g.mp && k >= 2 && k < g.lp) ka_bounds_cell<R, FIRST, STD, true>(P, A, i, j, k);
+  else ka_bounds_cell<R, FIRST, STD, false>(P, A, i, j, k);
 }
 
 // ---- pseudo-velocity (gauge): v = vdyf(xl,xr,a,hm) - 0.125*a*hm*cr ------------
@@ -357,8 +442,6 @@ __global__ void KA_LB_BOUNDS ka_bounds(const Prob<R> P, const AdjArr<R> A) {
 // AIN: a = the caller's Courant numbers (gradient into gu); otherwise a = the
 // previous pass's limited velocities, read with the wall rule (gradient into
 // that pass's lambda_w).
-template <class R> __device__ __forceinline__ R negv(R x) { return -x; }
-template <> __device__ __forceinline__ double negv<double>(double x) { return neg_bits(x); }
 
 // The adjoint of one face's v = K*(xr-xl) - 0.03125*a*hm*cr4, with
 // K = (|a| - a*a*hm)/2 and cr4 = S*D [+ S'*D'], the 4-face sums S times the
@@ -563,12 +646,132 @@ __global__ void KA_LB_PSEUDO ka_pseudo(const Prob<R> P, const AdjArr<R> A) {
   }
 }
 
+// The same reverse in gather form (FP32, every axis periodic): the scatter
+// above adds 57 values a cell by atomics, and at four bytes each the L2's
+// atomic rate bounds it.  The additions of a face go to cells and faces that
+// differ by a shift, so their sums over the two faces of a cell on each axis
+// are six cell-centred fields:
+//   T1 (T2, T3): R of the faces whose cross difference runs along x (y, z);
+//                lambda_x(i) gains T1(i-1) - T1(i+1), and so on
+//   C1 (C2, C3): the products on the 4-face sums of u1 (u2, u3);
+//                lambda_a1 of face i gains C1(i-1) + C1(i), and so on
+// A first kernel forms them (each face twice, once from either cell: FP64,
+// bound by its pipe, keeps the scatter) with what goes to the cell and its
+// lower faces themselves, a second one adds the shifted sums.  The pair sums
+// and velocity pairs come from kf_pairs, the six fields from the standard
+// form's accumulators.
+// 128x128x64: 44 + 14 us, 89 by scatter.
+template <class R, bool AIN, bool IN>
+__device__ __forceinline__ void ka_cross_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
+  const Geo& g = P.g;
+  const Arr<R>& U1 = AIN ? P.u1 : P.w1;
+  const Arr<R>& U2 = AIN ? P.u2 : P.w2;
+  const Arr<R>& U3 = AIN ? P.u3 : P.w3;
+  const int im = IN ? i - 1 : wrapi(i - 1, g.np), ip = IN ? i + 1 : wrapi(i + 1, g.np);
+  const int jm = IN ? j - 1 : wrapi(j - 1, g.mp), jp = IN ? j + 1 : wrapi(j + 1, g.mp);
+  const int km = IN ? k - 1 : wrapi(k - 1, g.lp), kp = IN ? k + 1 : wrapi(k + 1, g.lp);
+  const R x = P.xant.ld(i, j, k);
+  const R f1 = P.f1.ld(i, j, k), f2 = P.f2.ld(i, j, k), f3 = P.f3.ld(i, j, k);
+  R lx, C1, C2, C3, T1, T2, T3;
+  auto face = [&](const Arr<R>& LV, const Arr<R>& U, const Arr<R>& HM, int a, int b, int c, R xl, R xr_, R cr4) {
+    return FaceAdj<R, false>(LV.ld(a, b, c), U.ld(a, b, c), HM.ld(a, b, c), xl, xr_, cr4);
+  };
+  {  // x: cross differences along y and z
+    const R S2 = P.f2.ld(im, j, k) + f2, S3 = P.f3.ld(im, j, k) + f3;
+    const R D2 = P.cp.ld(i, jp, k) - P.cp.ld(i, jm, k), D3 = P.cp.ld(i, j, kp) - P.cp.ld(i, j, km);
+    const FaceAdj<R, false> f = face(A.lv1, U1, P.hmx, i, j, k, P.xant.ld(im, j, k), x, S2 * D2 + S3 * D3);
+    A.la1.at(i, j, k) += f.la;
+    C2 = f.lcr4 * D2;
+    T2 = f.lcr4 * S2;
+    C3 = f.lcr4 * D3;
+    T3 = f.lcr4 * S3;
+    lx = f.lK;
+  }
+  {
+    const R S2 = f2 + P.f2.ld(ip, j, k), S3 = f3 + P.f3.ld(ip, j, k);
+    const R D2 = P.cp.ld(ip, jp, k) - P.cp.ld(ip, jm, k), D3 = P.cp.ld(ip, j, kp) - P.cp.ld(ip, j, km);
+    const FaceAdj<R, false> f = face(A.lv1, U1, P.hmx, ip, j, k, x, x, R(0));
+    C2 += f.lcr4 * D2;
+    T2 += f.lcr4 * S2;
+    C3 += f.lcr4 * D3;
+    T3 += f.lcr4 * S3;
+    lx -= f.lK;
+  }
+  {  // y: along x and z
+    const R S1 = P.f1.ld(i, jm, k) + f1, S3 = P.f3.ld(i, jm, k) + f3;
+    const R D1 = P.cn.ld(ip, j, k) - P.cn.ld(im, j, k), D3 = P.cn.ld(i, j, kp) - P.cn.ld(i, j, km);
+    const FaceAdj<R, false> f = face(A.lv2, U2, P.hmy, i, j, k, P.xant.ld(i, jm, k), x, S1 * D1 + S3 * D3);
+    A.la2.at(i, j, k) += f.la;
+    C1 = f.lcr4 * D1;
+    T1 = f.lcr4 * S1;
+    C3 += f.lcr4 * D3;
+    T3 += f.lcr4 * S3;
+    lx += f.lK;
+  }
+  {
+    const R S1 = f1 + P.f1.ld(i, jp, k), S3 = f3 + P.f3.ld(i, jp, k);
+    const R D1 = P.cn.ld(ip, jp, k) - P.cn.ld(im, jp, k), D3 = P.cn.ld(i, jp, kp) - P.cn.ld(i, jp, km);
+    const FaceAdj<R, false> f = face(A.lv2, U2, P.hmy, i, jp, k, x, x, R(0));
+    C1 += f.lcr4 * D1;
+    T1 += f.lcr4 * S1;
+    C3 += f.lcr4 * D3;
+    T3 += f.lcr4 * S3;
+    lx -= f.lK;
+  }
+  {  // z: along x and y
+    const R S1 = P.f1.ld(i, j, km) + f1, S2 = P.f2.ld(i, j, km) + f2;
+    const R D1 = P.q.ld(ip, j, k) - P.q.ld(im, j, k), D2 = P.q.ld(i, jp, k) - P.q.ld(i, jm, k);
+    const FaceAdj<R, false> f = face(A.lv3, U3, P.hmz, i, j, k, P.xant.ld(i, j, km), x, S1 * D1 + S2 * D2);
+    A.la3.at(i, j, k) += f.la;
+    C1 += f.lcr4 * D1;
+    T1 += f.lcr4 * S1;
+    C2 += f.lcr4 * D2;
+    T2 += f.lcr4 * S2;
+    lx += f.lK;
+  }
+  {
+    const R S1 = f1 + P.f1.ld(i, j, kp), S2 = f2 + P.f2.ld(i, j, kp);
+    const R D1 = P.q.ld(ip, j, kp) - P.q.ld(im, j, kp), D2 = P.q.ld(i, jp, kp) - P.q.ld(i, jm, kp);
+    const FaceAdj<R, false> f = face(A.lv3, U3, P.hmz, i, j, kp, x, x, R(0));
+    C1 += f.lcr4 * D1;
+    T1 += f.lcr4 * S1;
+    C2 += f.lcr4 * D2;
+    T2 += f.lcr4 * S2;
+    lx -= f.lK;
+  }
+  A.lxant.at(i, j, k) += lx;
+  A.lg1.at(i, j, k) = C1;
+  A.lg2.at(i, j, k) = C2;
+  A.lg3.at(i, j, k) = C3;
+  A.lf1.at(i, j, k) = T1;
+  A.lf2.at(i, j, k) = T2;
+  A.lf3.at(i, j, k) = T3;
+}
+template <class R, bool AIN>
+__global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R> A) {
+#define C(IN) ka_cross_cell<R, AIN, IN>(P, A, i, j, k)
+  ADISPATCH(C)
+#undef C
+}
+template <class R>
+__global__ void __launch_bounds__(128) ka_cross_sum(const Prob<R> P, const AdjArr<R> A) {
+  ACELL
+  const int im = wrapi(i - 1, g.np), ip = wrapi(i + 1, g.np), jm = wrapi(j - 1, g.mp), jp = wrapi(j + 1, g.mp),
+            km = wrapi(k - 1, g.lp), kp = wrapi(k + 1, g.lp);
+  A.lxant.at(i, j, k) += (A.lf1.ld(im, j, k) - A.lf1.ld(ip, j, k)) + (A.lf2.ld(i, jm, k) - A.lf2.ld(i, jp, k)) +
+                         (A.lf3.ld(i, j, km) - A.lf3.ld(i, j, kp));
+  A.la1.at(i, j, k) += A.lg1.ld(im, j, k) + A.lg1.ld(i, j, k);
+  A.la2.at(i, j, k) += A.lg2.ld(i, jm, k) + A.lg2.ld(i, j, k);
+  A.la3.at(i, j, k) += A.lg3.ld(i, j, km) + A.lg3.ld(i, j, k);
+}
+
 // ---- standard form (antidiff3d-standard-gpubc.f90) ---------------------------
 // update: x_out = rhr*(q - d*hinv), d = signed sum of the limited fluxes g
 template <class R, bool IN>
 __device__ __forceinline__ void ka_update_std_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
   const Geo& g = P.g;
   const R lt = P.rhr.ld(i, j, k) * A.lam.ld(i, j, k);
+  if (A.lx.p) A.lx.at(i, j, k) = R(0);  // as the gauge form's update
   addat(A.lq, i, j, k, lt);
   const R lD = -lt * P.hinv.ld(i, j, k);
   fx_add<R, false, IN>(g, A.lg1, i + 1, j, k, lD);
@@ -774,84 +977,110 @@ __global__ void __launch_bounds__(128) ka_pseudo_std(const Prob<R> P, const AdjA
 // ---- upwind: xant = rhr*(x - D*hinv), D = signed sum of donor fluxes --------
 // F = donor(xl, xr, u) = pp(u)*xl - pn(u)*xr; dF/du = [u>0]*xl + [u<0]*xr.
 // Open-wall neighbours come from bcx/bcy (constants: no gradient).
+//
+// A cell owns its lower face on each axis (the last cell of an open axis the
+// upper one as well) and forms that face's lambda_F from both of its cells:
+// three fluxes a cell instead of six, one atomic each (the donor cell's), the
+// velocity gradient by a plain read and write.  256x256x64 FP64: 142 us, half
+// of it the FP64 pipe's; six fluxes from a cell and a copy of the result 167.
+// MF (density step): the step also outputs each face's upwind flux as part
+// of its mass flux: the lower face's flux of every cell (u1(i), u2(j), u3(k))
+// and the upper face's of the last cell along each axis (u1(np+1), ...),
+// which a periodic axis takes from face 1.  Their cotangents add to the
+// fluxes' own; at a z wall the flux stored for face 1 is -F3(2) and the one
+// for face lp+1 is -F3(lp).
 template <class R>
-__device__ __forceinline__ void flux_adj(R lF, R xl, R xr_, R u, bool l_var, const Arr<R>& Lx, int li, int lj,
-                                         int lk, bool r_var, int ri, int rj, int rk, R* lu_out) {
-  // F = pp(u)*xl - pn(u)*xr: dF/dxl = pp(u), dF/dxr = -pn(u) (one of them
-  // is u, the other zero), dF/du = dpp(u)*xl - dpn(u)*xr
+__device__ __forceinline__ void flux_adj(R lF, R u, R xl, R xr_, R* GU, const Arr<R>& Lx, bool l_var, int li, int lj,
+                                         int lk, bool r_var, int ri, int rj, int rk) {
   const R m = lF * u;
   if (sgn(u)) {
     if (r_var) addat(Lx, ri, rj, rk, m);
   } else {
     if (l_var) addat(Lx, li, lj, lk, m);
   }
-  *lu_out = nonzero(u) ? lF * (sgn(u) ? xr_ : xl) : R(0);
+  if (nonzero(u)) *GU += lF * (sgn(u) ? xr_ : xl);
 }
 
-// MF (density step): the step also outputs each face's upwind flux as part
-// of its mass flux: the lower face's flux of every cell (u1(i), u2(j), u3(k))
-// and the upper face's of the last cell along each axis (u1(np+1), ...).
-// Their cotangents add to the fluxes' own; at a z wall the flux stored for
-// face 1 is -F3(2) and the one for face lp+1 is -F3(lp).
-template <class R, bool IN, bool MF = false>
+// U: rhr and hinv are exactly 1 at the cells read (x*1 == x); an instantiation,
+// as a test inside the body became selects between products computed anyway.
+template <class R, bool IN, bool MF, bool U>
 __device__ __forceinline__ void ka_upwind_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
   const Geo& g = P.g;
   const Arr<R>& psi = P.psi;
-  const R lxa = A.lxant.ld(i, j, k);
-  const R rh = P.rhr.ld(i, j, k);
-  addat(A.lx, i, j, k, lxa * rh);
-  const R lD = -lxa * rh * P.hinv.ld(i, j, k);
-  const R x = psi.ld(i, j, k);
+  // the adjoint of a cell's divergence
+  auto div = [&](int a, int b, int c) {
+    const R l = negv(A.lxant.ld(a, b, c));
+    return U ? l : l * P.rhr.ld(a, b, c) * P.hinv.ld(a, b, c);
+  };
+  {
+    const R l = A.lxant.ld(i, j, k);
+    addat(A.lx, i, j, k, U ? l : l * P.rhr.ld(i, j, k));
+  }
+  const R lD = div(i, j, k), x = psi.ld(i, j, k);
   const long bx0 = (long)(j - 1) + (long)g.mp * (k - 1), bxs = (long)g.mp * g.lp;
   const long by0 = (long)(i - 1) + (long)g.np * (k - 1), bys = (long)g.np * g.lp;
-  const bool im_var = IN || i > 1 || g.bx, ip_var = IN || i < g.np || g.bx, jm_var = IN || j > 1 || g.by, jp_var = IN || j < g.mp || g.by;
-  const int im = IN ? i - 1 : wrapi(i - 1, g.np), ip = IN ? i + 1 : wrapi(i + 1, g.np), jm = IN ? j - 1 : wrapi(j - 1, g.mp), jp = IN ? j + 1 : wrapi(j + 1, g.mp);
-  const R xim = im_var ? psi.ld(im, j, k) : P.bcx[bx0];
-  const R xip = ip_var ? psi.ld(ip, j, k) : P.bcx[bx0 + bxs];
-  const R xjm = jm_var ? psi.ld(i, jm, k) : P.bcy[by0];
-  const R xjp = jp_var ? psi.ld(i, jp, k) : P.bcy[by0 + bys];
-  R lu;
-  // the mass fluxes' cotangents of the fluxes this cell computes (MF)
-  R m1 = R(0), m1p = R(0), m2 = R(0), m2p = R(0), m3 = R(0), m3p = R(0);
-  if (MF) {
-    m1 = A.lm1.ld(i, j, k);
-    m2 = A.lm2.ld(i, j, k);
-    m3 = A.lm3.ld(i, j, k);
-    if (!IN && i == g.np) m1p = A.lm1.ld(g.np + 1, j, k);
-    if (!IN && j == g.mp) m2p = A.lm2.ld(i, g.mp + 1, k);
-    if (!IN && k == g.lp) m3p = A.lm3.ld(i, j, g.lp + 1);
+  {
+    const bool var = IN || i > 1 || g.bx;
+    const int im = IN ? i - 1 : wrapi(i - 1, g.np);
+    R lF = (var ? div(im, j, k) : R(0)) - lD;
+    if (MF) {
+      lF += A.lm1.ld(i, j, k);
+      if (!IN && i == 1 && g.bx) lF += A.lm1.ld(g.np + 1, j, k);
+    }
+    flux_adj(lF, P.u1.ld(i, j, k), var ? psi.ld(im, j, k) : P.bcx[bx0], x, &A.gu1.at(i, j, k), A.lx, var, im, j, k,
+             true, i, j, k);
+    if (!IN && i == g.np && !g.bx)
+      flux_adj(MF ? lD + A.lm1.ld(i + 1, j, k) : lD, P.u1.ld(i + 1, j, k), x, P.bcx[bx0 + bxs],
+               &A.gu1.at(i + 1, j, k), A.lx, true, i, j, k, false, i, j, k);
   }
-  // x faces: D = F1(i+1) - F1(i) + ...
-  flux_adj(lD + m1p, x, xip, fx<R, true, IN>(g, P.u1, i + 1, j, k), true, A.lx, i, j, k, ip_var, ip, j, k, &lu);
-  fx_add<R, true, IN>(g, A.gu1, i + 1, j, k, lu);
-  flux_adj(-lD + m1, xim, x, P.u1.ld(i, j, k), im_var, A.lx, im, j, k, true, i, j, k, &lu);
-  fx_add<R, true, IN>(g, A.gu1, i, j, k, lu);
-  flux_adj(lD + m2p, x, xjp, fy<R, true, IN>(g, P.u2, i, j + 1, k), true, A.lx, i, j, k, jp_var, i, jp, k, &lu);
-  fy_add<R, true, IN>(g, A.gu2, i, j + 1, k, lu);
-  flux_adj(-lD + m2, xjm, x, P.u2.ld(i, j, k), jm_var, A.lx, i, jm, k, true, i, j, k, &lu);
-  fy_add<R, true, IN>(g, A.gu2, i, j, k, lu);
-  if (!IN && !g.bz && k == 1) {  // F3(1) = -F3(2): D = ... + 2*F3(2); the flux stored for face 1 is -F3(2)
-    flux_adj(R(2) * lD - m3, x, psi.ld(i, j, k + 1), P.u3.ld(i, j, k + 1), true, A.lx, i, j, k, true, i, j, k + 1,
-             &lu);
-    addat(A.gu3, i, j, k + 1, lu);
-  } else if (!IN && !g.bz && k == g.lp) {  // F3(lp+1) = -F3(lp): D = ... - 2*F3(lp); face lp+1 stores -F3(lp)
-    flux_adj(-R(2) * lD + m3 - m3p, psi.ld(i, j, k - 1), x, P.u3.ld(i, j, k), true, A.lx, i, j, k - 1, true, i, j,
-             k, &lu);
-    addat(A.gu3, i, j, k, lu);
-  } else {
-    const int kp = cz<IN>(g, k + 1), km = cz<IN>(g, k - 1);
-    flux_adj(lD + m3p, x, psi.ld(i, j, kp), fz<R, true, IN>(g, P.u3, i, j, k + 1), true, A.lx, i, j, k, true, i,
-             j, kp, &lu);
-    fz_add<R, true, IN>(g, A.gu3, i, j, k + 1, lu);
-    flux_adj(-lD + m3, psi.ld(i, j, km), x, P.u3.ld(i, j, k), true, A.lx, i, j, km, true, i, j, k, &lu);
-    fz_add<R, true, IN>(g, A.gu3, i, j, k, lu);
+  {
+    const bool var = IN || j > 1 || g.by;
+    const int jm = IN ? j - 1 : wrapi(j - 1, g.mp);
+    R lF = (var ? div(i, jm, k) : R(0)) - lD;
+    if (MF) {
+      lF += A.lm2.ld(i, j, k);
+      if (!IN && j == 1 && g.by) lF += A.lm2.ld(i, g.mp + 1, k);
+    }
+    flux_adj(lF, P.u2.ld(i, j, k), var ? psi.ld(i, jm, k) : P.bcy[by0], x, &A.gu2.at(i, j, k), A.lx, var, i, jm, k,
+             true, i, j, k);
+    if (!IN && j == g.mp && !g.by)
+      flux_adj(MF ? lD + A.lm2.ld(i, j + 1, k) : lD, P.u2.ld(i, j + 1, k), x, P.bcy[by0 + bys],
+               &A.gu2.at(i, j + 1, k), A.lx, true, i, j, k, false, i, j, k);
+  }
+  if (IN || g.bz || k > 1) {
+    const int km = IN ? k - 1 : wrapi(k - 1, g.lp);
+    const bool wall = !g.bz;
+    const R dl = div(i, j, km);
+    // F3(1) = -F3(2) and F3(lp+1) = -F3(lp): a wall cell reads its inner face twice
+    R lF = (wall && k == 2 ? scale_up<1>(dl) : dl) - (wall && k == g.lp ? scale_up<1>(lD) : lD);
+    if (MF) {
+      lF += A.lm3.ld(i, j, k);
+      if (wall && k == 2) lF -= A.lm3.ld(i, j, 1);
+      if (!IN && wall && k == g.lp) lF -= A.lm3.ld(i, j, g.lp + 1);
+      if (!IN && g.bz && k == 1) lF += A.lm3.ld(i, j, g.lp + 1);
+    }
+    flux_adj(lF, P.u3.ld(i, j, k), psi.ld(i, j, km), x, &A.gu3.at(i, j, k), A.lx, true, i, j, km, true, i, j, k);
   }
 }
 template <class R, bool MF = false>
 __global__ void KA_LB_UPWIND ka_upwind(const Prob<R> P, const AdjArr<R> A) {
-#define C(IN) ka_upwind_cell<R, IN, MF>(P, A, i, j, k)
-  ADISPATCH(C)
-#undef C
+  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const int k = blockIdx.z + 1;
+  const bool win = warp_interior(P.g, i, j, k);
+  if (i > P.g.np || j > P.g.mp) return;
+  if (!win) {
+    ka_upwind_cell<R, false, MF, false>(P, A, i, j, k);
+    return;
+  }
+  if constexpr (sizeof(R) == 8) {
+    auto one = [&](int a, int b, int c) { return is_one(P.rhr.ld(a, b, c)) && is_one(P.hinv.ld(a, b, c)); };
+    if (__all_sync(0xffffffffu, one(i, j, k) && one(i - 1, j, k) && one(i, j - 1, k) && one(i, j, k - 1))) {
+      ka_upwind_cell<R, true, MF, true>(P, A, i, j, k);
+      return;
+    }
+  }
+  ka_upwind_cell<R, true, MF, false>(P, A, i, j, k);
 }
 
 // Density step: the mass flux of every face adds the last pass's limited
@@ -889,12 +1118,6 @@ __global__ void __launch_bounds__(128) ka_rho_out(const Prob<R> P, const Arr<R> 
   lam.at(i, j, k) = lam.ld(i, j, k) + l_xc * h;
   g_xinc.at(i, j, k) = quot(a_rh, xc);
   g_pexe.at(i, j, k) = a_p1 * xc;
-}
-
-template <class R>
-__global__ void __launch_bounds__(128) ka_store(const Prob<R> P, const AdjArr<R> A) {
-  ACELL
-  A.lam.at(i, j, k) = A.lx.ld(i, j, k);
 }
 
 // J's seed: lambda = psi_N - target on the interior, 0 on the halo.
@@ -1106,6 +1329,10 @@ int run_step_record(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<
     else if (!keep) kf_bounds<R, true, true, false><<<grd, blk, 0, s>>>(Q);
     else if (t == 0) kf_bounds<R, true, true, true><<<grd, blk, 0, s>>>(Q);
     else kf_bounds<R, true, false, true><<<grd, blk, 0, s>>>(Q);
+    n += 2;
+    // only the update and the next pass read the limited velocities: the last
+    // pass of a step whose output is not wanted leaves them out
+    if (t == np_ - 1 && !out) break;
     // the limited fluxes (standard form) go to the workspace scratch: only
     // the update reads them
     Prob<R> L = Q;
@@ -1114,13 +1341,10 @@ int run_step_record(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<
     L.f3 = P.f3;
     if (nonos) kf_limit<R, true><<<grd, blk, 0, s>>>(L);
     else kf_limit<R, false><<<grd, blk, 0, s>>>(L);
-    n += 3;
-    if (t < np_ - 1 || out) {
-      Prob<R> U = L;
-      U.xant = t < np_ - 1 ? A.x[t + 1] : *out;
-      kf_update<R><<<grd, blk, 0, s>>>(U);
-      n++;
-    }
+    Prob<R> U = L;
+    U.xant = t < np_ - 1 ? A.x[t + 1] : *out;
+    kf_update<R><<<grd, blk, 0, s>>>(U);
+    n += 2;
   }
   add_launches(n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
@@ -1135,8 +1359,22 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
   const int np_ = A.npass;
   int n = 0;
-  if (cudaMemsetAsync(A.acc, 0, A.acc_elems * sizeof(R), s) != cudaSuccess) return -5;
-  if (A.rho && A.lm1.p) {  // the density step's mass fluxes read the last pass's limited fluxes
+  // The accumulators that kernels add to.  Standard form: all of them.  Gauge
+  // form: lambda_w of every pass but the last (the next pass's pseudo-velocity
+  // adds to it), and of the last where mass fluxes have cotangents; with the
+  // limiter lcp and lcn, and the running extrema of every pass but the last.
+  // Every other array is stored whole by the first kernel that writes it.
+  const bool mass = A.rho && A.lm1.p;
+  const size_t n1 = A.pass_acc_elems / 12;  // elements of one field
+  auto zero = [&](R* p, size_t fields) { return cudaMemsetAsync(p, 0, fields * n1 * sizeof(R), s) == cudaSuccess; };
+  if (P.stdf) {
+    if (cudaMemsetAsync(A.acc, 0, A.acc_elems * sizeof(R), s) != cudaSuccess) return -5;
+  } else {  // a pass's six: lx, lw*3, lmx, lmn
+    for (int t = 0; t < np_ - 1; t++)
+      if (!zero(A.acc + (6 * t + 1) * n1, 5)) return -5;
+    if (mass && !zero(A.acc + (6 * (np_ - 1) + 1) * n1, 3)) return -5;
+  }
+  if (mass) {  // the density step's mass fluxes read the last pass's limited fluxes
     AdjArr<R> m{};
     m.lw1 = A.lw[np_ - 1][0];
     m.lw2 = A.lw[np_ - 1][1];
@@ -1149,7 +1387,8 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
   }
   // ---- reverse, last pass first
   for (int t = np_ - 1; t >= 0; t--) {
-    if (t < np_ - 1 && cudaMemsetAsync(A.pass_acc, 0, A.pass_acc_elems * sizeof(R), s) != cudaSuccess) return -5;
+    if (P.stdf && t < np_ - 1 && !zero(A.pass_acc, 12)) return -5;
+    if (!P.stdf && nonos && !zero(A.pass_acc + 3 * n1, 2)) return -5;  // lcp, lcn
     const Prob<R> Q = pass_prob(P, A, t, true);
     AdjArr<R> a{};
     a.lxant = A.lx[t];
@@ -1161,7 +1400,7 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
     a.lw3 = A.lw[t][2];
     a.lcp = A.lcp;
     a.lcn = A.lcn;
-    a.lx = A.lxin;
+    a.lx = A.lam;  // once the last pass's update has read the caller's lambda
     a.lam = t == np_ - 1 ? A.lam : A.lx[t + 1];
     a.gu1 = A.gu1;
     a.gu2 = A.gu2;
@@ -1182,8 +1421,10 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
     a.lf2 = A.lf[1];
     a.lf3 = A.lf[2];
     a.lq = A.lq;
+    AdjArr<R> au = a;
+    if (t < np_ - 1) au.lx.p = nullptr;
     if (P.stdf) {
-      ka_update_std<R><<<grd, blk, 0, s>>>(Q, a);
+      ka_update_std<R><<<grd, blk, 0, s>>>(Q, au);
       if (nonos) {
         ka_limit_std<R, true><<<grd, blk, 0, s>>>(Q, a);
         if (t == 0) ka_bounds<R, true, true><<<grd, blk, 0, s>>>(Q, a);
@@ -1195,7 +1436,11 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
       if (t == 0) ka_pseudo_std<R, true><<<grd, blk, 0, s>>>(Q, a);
       else ka_pseudo_std<R, false><<<grd, blk, 0, s>>>(Q, a);
     } else {
-      ka_update<R><<<grd, blk, 0, s>>>(Q, a);
+      if (t == np_ - 1) {  // nothing carried back, nothing added to lambda_w
+        a.lmx.p = a.lmn.p = nullptr;
+        if (!mass) a.lw1.p = a.lw2.p = a.lw3.p = nullptr;
+      }
+      ka_update<R><<<grd, blk, 0, s>>>(Q, au);
       if (nonos) {
         ka_limit<R, true><<<grd, blk, 0, s>>>(Q, a);
         if (t == 0) ka_bounds<R, true, false><<<grd, blk, 0, s>>>(Q, a);
@@ -1217,18 +1462,27 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
         else kf_pairs<R, false, true><<<grd, blk, 0, s>>>(Qp);
         n++;
       }
-      if (t == 0) ka_pseudo<R, true><<<grd, blk, 0, s>>>(Qp, a);
-      else ka_pseudo<R, false><<<grd, blk, 0, s>>>(Qp, a);
+      if (sizeof(R) == 4 && g.bx && g.by && g.bz) {
+        if constexpr (sizeof(R) == 4) {
+          if (t == 0) ka_cross<R, true><<<grd, blk, 0, s>>>(Qp, a);
+          else ka_cross<R, false><<<grd, blk, 0, s>>>(Qp, a);
+          ka_cross_sum<R><<<grd, blk, 0, s>>>(Qp, a);
+          n++;
+        }
+      } else if (t == 0) {
+        ka_pseudo<R, true><<<grd, blk, 0, s>>>(Qp, a);
+      } else {
+        ka_pseudo<R, false><<<grd, blk, 0, s>>>(Qp, a);
+      }
     }
     n += 3;
   }
   AdjArr<R> a0{};
   a0.lxant = A.lx[0];
-  a0.lx = A.lxin;
+  a0.lx = A.lam;
   a0.gu1 = A.gu1;
   a0.gu2 = A.gu2;
   a0.gu3 = A.gu3;
-  a0.lam = A.lam;
   if (A.rho && A.lm1.p) {
     a0.lm1 = A.lm1;
     a0.lm2 = A.lm2;
@@ -1237,8 +1491,7 @@ int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStrea
   } else {
     ka_upwind<R><<<grd, blk, 0, s>>>(P, a0);
   }
-  ka_store<R><<<grd, blk, 0, s>>>(P, a0);
-  n += 2;
+  n++;
   add_launches(n);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -1502,7 +1502,7 @@ int rho_adjoint_impl(void* ws, const R* u1, const R* u2, const R* u3, const R* x
     P.rho = 1;
     P.x_incomp = caller_view<R>(const_cast<R*>(x_incomp), ih, sx, sy);
     P.pexe = caller_view<R>(const_cast<R*>(pexe), ih, sx, sy);
-    P.rhoadv = A.lq;  // the recorded upwind copies x_incomp there; the reverse clears it
+    P.rhoadv = A.lq;  // the recorded upwind copies x_incomp there; the reverse writes it anew
     R* hi = static_cast<R*>(w->mem) + (size_t)NSCRATCH * w->ncell;
     P.f1hi = hi;
     P.f2hi = hi + (size_t)g.mp * g.lp;
