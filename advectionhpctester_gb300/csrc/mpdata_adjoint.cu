@@ -1350,6 +1350,25 @@ int run_step_record(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
+int run_record_ratios(const Prob<float>& P, const AdjPlan<float>& A, cudaStream_t s) {
+  const Geo& g = P.g;
+  const dim3 blk(32, 4, 1);
+  const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
+  kf_bounds<float, true, true, false><<<grd, blk, 0, s>>>(pass_prob(P, A, 0, false));
+  add_launches(1);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+int run_record_reciprocals(const Prob<float>& P, const AdjPlan<float>& A, cudaStream_t s) {
+  const Geo& g = P.g;
+  const dim3 blk(32, 4, 1);
+  const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
+  Prob<float> F = P;
+  F.xant = A.x[0];  // the upwind field comes with them
+  kf_upwind<float><<<grd, blk, 0, s>>>(F);
+  add_launches(1);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
 // The reverse kernels of one recorded step: lambda of the step's output (A.lam)
 // becomes lambda of its input; the velocity gradients accumulate into A.gu*.
 template <class R>

@@ -167,27 +167,33 @@ Prob<R> make_prob(const mpdata_grid& g, int gauge, R* psi, const R* u1, const R*
   return P;
 }
 
+// The fused step's arguments for the problem P.
+FusedPlan fused_plan(const Prob<float>& P, float* arena, int kchunk, int* err, const CUtensorMap* map) {
+  FusedPlan F;
+  F.g = P.g;
+  F.cls = fused_class(P.g, !P.stdf);
+  F.bcx = P.bcx;
+  F.bcy = P.bcy;
+  F.psi = P.psi;
+  F.u1 = P.u1;
+  F.u2 = P.u2;
+  F.u3 = P.u3;
+  F.h = P.h;
+  F.rhr = P.rhr;
+  F.arena = arena;
+  F.kchunk = kchunk;
+  F.err = err;
+  F.tmap = map;
+  return F;
+}
+
 // One step of the workspace's problem P: the fused single-precision kernels
 // when the workspace qualifies, else the stage kernels (same bits).
 template <class R>
 int ws_step(Workspace* w, const Prob<R>& P, Prof* prof, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
     if (w->fused) {
-      FusedPlan F;
-      F.g = P.g;
-      F.cls = fused_class(P.g, !P.stdf);
-      F.bcx = P.bcx;
-      F.bcy = P.bcy;
-      F.psi = P.psi;
-      F.u1 = P.u1;
-      F.u2 = P.u2;
-      F.u3 = P.u3;
-      F.h = P.h;
-      F.rhr = P.rhr;
-      F.arena = static_cast<float*>(w->mem);
-      F.kchunk = w->fz_kchunk;
-      F.err = w->d_err;
-      F.tmap = &w->fz_map;
+      const FusedPlan F = fused_plan(P, static_cast<float*>(w->mem), w->fz_kchunk, w->d_err, &w->fz_map);
       w->fz_extrema = true;
       return run_step_fused(F, w->o.iord, prof, s, &w->fz_mx, &w->fz_mn) == 0 ? MPDATA_OK : MPDATA_E_CUDA;
     }
@@ -1335,6 +1341,11 @@ int step_adjoint_impl(void* ws, const R* psi_in, const R* u1, const R* u2, const
 // kernels read those records, so each step runs forward twice instead of
 // three times.  Peak extra memory: (checkpoints + interval) psi-sized arrays,
 // plus (interval - 1) record arenas when they are kept.
+// FP32 gauge steps of one corrective pass are recorded by the fused step's
+// kernels, each into an arena of its own (the interval's number of them), and
+// the ratios by one more kernel; the forward sweep records the last segment as
+// it goes, so that its steps run forward once.  128x128x64, a step's record
+// with its output: 90 us, 127 by the stage kernels.
 template <class R>
 int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, const R* u2, const R* u3,
                      const R* h, const R* rhr, const R* bcx, const R* bcy, const R* target, double* J,
@@ -1371,25 +1382,48 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
     if (seg) cudaFreeAsync(seg, s);
     return MPDATA_E_CUDA;
   }
-  // one record arena per step of a segment (the workspace's own is the first)
+  // one record arena per step of a segment (of the stage kernels' ones the
+  // workspace's own is the first)
   const size_t nrec = adj_record_fields(w->o.iord);
-  const size_t rec_bytes = nrec * w->ncell * w->elem;
+  const FusedArena fa = fused_arena(P.g);
+  const size_t fz_flags = (size_t)FZ_NREC * fa.fs, fz_tail = fz_flags + ((size_t)fa.ntx * fa.nty * P.g.lp + 3) / 4;
+  const size_t fz_elems = (fz_tail + 3 * w->ncell + 63) / 64 * 64;
+  bool fz = sizeof(R) == 4 && K > 1 && w->fused && w->o.gauge && w->o.iord == 2;
+  const size_t rec_bytes = fz ? fz_elems * sizeof(R) : nrec * w->ncell * w->elem;
+  const size_t nrecs = fz ? K : K - 1;
   R* recs = nullptr;
   {
     size_t free_b = 0, total_b = 0;
-    if (K > 1 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && (size_t)(K - 1) * rec_bytes < free_b / 2 &&
-        cudaMallocAsync(&recs, (size_t)(K - 1) * rec_bytes, s) != cudaSuccess) {
+    if (K > 1 && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && nrecs * rec_bytes < free_b / 2 &&
+        cudaMallocAsync(&recs, nrecs * rec_bytes, s) != cudaSuccess) {
       cudaGetLastError();
       recs = nullptr;
     }
   }
   std::vector<AdjPlan<R>> plans;
+  std::vector<CUtensorMap> maps;
+  fz = fz && recs;
   if (recs) {
     plans.assign((size_t)K, A);
-    for (int k = 1; k < K; k++) repoint_records<R>(&plans[k], recs + (size_t)(k - 1) * nrec * w->ncell, w->ncell, P.g);
+    if constexpr (sizeof(R) == 4) {
+      if (fz) {
+        maps.resize((size_t)K);
+        for (int k = 0; k < K && !rc; k++) {
+          R* a = recs + (size_t)k * fz_elems;
+          if (fused_make_tmap(&maps[k], a, P.g, FZ_NREC)) rc = MPDATA_E_CUDA;
+          plans[k].x[0] = fused_view(a, FZ_X0, P.g);
+          for (int c = 0; c < 3; c++) plans[k].v[0][c] = fused_view(a, FZ_V1 + c, P.g);
+          Arr<R>* const ratios[3] = {&plans[k].cp[0], &plans[k].cn[0], &plans[k].q[0]};
+          for (int c = 0; c < 3; c++) *ratios[c] = scratch_view<R>(a + fz_tail + (size_t)c * w->ncell, P.g);
+        }
+      }
+    }
+    if (!fz)
+      for (int k = 1; k < K; k++)
+        repoint_records<R>(&plans[k], recs + (size_t)(k - 1) * nrec * w->ncell, w->ncell, P.g);
   }
   if (peak_bytes)
-    *peak_bytes = (long long)(pbytes * (nck + K)) + (long long)(recs ? (size_t)(K - 1) * rec_bytes : 0) +
+    *peak_bytes = (long long)(pbytes * (nck + K)) + (long long)(recs ? nrecs * rec_bytes : 0) +
                   (long long)(w->ncell * w->elem * (NSCRATCH + nrec + adj_acc_fields(w->o.iord)));
   R* base = static_cast<R*>(w->mem);
   auto fwd = [&](R* state) -> int {
@@ -1397,12 +1431,41 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
                              base + (size_t)NFIELD * w->ncell, 1);
     return ws_step<R>(w, F, nullptr, s);
   };
+  // record of a segment's step (slot) from its state src; the next state, when
+  // it is wanted, into dst (fused records)
+  auto record = [&](int slot, R* src, R* dst) -> int {
+    if constexpr (sizeof(R) == 4) {
+      Prob<R> B = P;
+      B.psi = caller_view<R>(dst ? dst : src, ih, sx, sy);
+      R* const a = recs + (size_t)slot * fz_elems;
+      FusedPlan F = fused_plan(B, a, w->fz_kchunk, w->d_err, &maps[slot]);
+      F.flags = reinterpret_cast<unsigned char*>(a + fz_flags);
+      if (dst && cudaMemcpyAsync(dst, src, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return MPDATA_E_CUDA;
+      if (run_record_fused(F, dst != nullptr, s)) return MPDATA_E_CUDA;
+      B.psi = caller_view<R>(src, ih, sx, sy);
+      return run_record_ratios(B, plans[slot], s) ? MPDATA_E_CUDA : MPDATA_OK;
+    }
+    return MPDATA_E_UNSUPPORTED;
+  };
   // forward sweep with checkpoints
-  for (int n = 0; n < nsteps && !rc; n++) {
+  const int n_last = (nck - 1) * K;  // the last segment, recorded on the way by the fused kernels
+  for (int n = 0; n < (fz ? n_last : nsteps) && !rc; n++) {
     if (n % K == 0 &&
         cudaMemcpyAsync(ck + (size_t)(n / K) * plen, psi, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
       rc = MPDATA_E_CUDA;
     if (!rc && fwd(psi)) rc = MPDATA_E_CUDA;
+  }
+  if constexpr (sizeof(R) == 4) {
+    if (fz && !rc) {
+      if (cudaMemcpyAsync(seg, psi, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) rc = MPDATA_E_CUDA;
+      for (int n = n_last; n < nsteps && !rc; n++) {
+        R* const src = seg + (size_t)(n - n_last) * plen;
+        rc = record(n - n_last, src, n + 1 < nsteps ? src + plen : psi);
+      }
+      w->fz_extrema = true;
+      w->fz_mx = w->fz_mn = -1;
+      if (!rc && run_record_reciprocals(P, A, s)) rc = MPDATA_E_CUDA;
+    }
   }
   // J and the seed lambda = psi_N - target (into g_psi0)
   double out[4] = {0, 0, 0, 0};
@@ -1416,14 +1479,19 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
   // reverse sweep, segment by segment
   for (int c = nck - 1; c >= 0 && !rc; c--) {
     const int n0 = c * K, n1 = (n0 + K < nsteps) ? n0 + K : nsteps;
-    if (cudaMemcpyAsync(seg, ck + (size_t)c * plen, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
+    const bool made = fz && c == nck - 1;  // the forward sweep left this segment's states and records
+    if (!made && cudaMemcpyAsync(seg, ck + (size_t)c * plen, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
       rc = MPDATA_E_CUDA;
       break;
     }
     if (recs) {
       // records of every step of the segment, each step's output into the next state
-      for (int n = n0; n < n1 && !rc; n++) {
+      for (int n = n0; n < n1 && !rc && !made; n++) {
         R* src = seg + (size_t)(n - n0) * plen;
+        if (fz) {
+          rc = record(n - n0, src, n + 1 < n1 ? src + plen : nullptr);
+          continue;
+        }
         Prob<R> B = P;
         B.psi = caller_view<R>(src, ih, sx, sy);
         const bool more = n + 1 < n1;  // the segment's last output is the next checkpoint

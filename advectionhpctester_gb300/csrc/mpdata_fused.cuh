@@ -48,6 +48,7 @@ struct FusedPlan {
   int kchunk;   // planes per block of the z-march
   int* err;     // device error word (bit 1: a staging wait timed out)
   const CUtensorMap* tmap;  // one 4-D map over the arena (x, y, z, field)
+  unsigned char* flags = nullptr;  // the unit flags, where they do not follow the FZ_NF fields
 };
 
 // Whether a step takes the fused path: FP32, nonoscillatory, iord >= 2, not the
@@ -65,13 +66,20 @@ FusedArena fused_arena(const Geo& g);
 // An arena field's interior as an array view.
 Arr<float> fused_view(float* arena, int field, const Geo& g);
 // Encodes the arena's tensor map (box 72 x 20 x 1 x 1).  0 on success.
-int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g);
+int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g, int fields = FZ_NF);
 // Planes per block of the z-march for each of the n grids that one launch
 // covers (MPDATA_FUSED_KCHUNK overrides).
 void fused_kchunk(const Geo* g, int n, int* kchunk);
 // One step; on return *mx_field / *mn_field name the arena fields that hold
 // the running extrema of the step (-1 when iord = 2 keeps none).
 int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int* mx_field, int* mn_field);
+
+// The forward record of an iord-2 gauge step, left in the arena F names: the
+// fields up to FZ_V3 (FZ_NREC of them, and the flags), of which FZ_X0 holds the
+// upwind field and FZ_V1..3 the pseudo-velocities.  update: the step's output is
+// written to F.psi as by run_step_fused; without it only the record is made.
+constexpr int FZ_NREC = FZ_V3 + 1;
+int run_record_fused(const FusedPlan& F, bool update, cudaStream_t s);
 
 // Batches.  Each problem of the fused table gets work items (a tile and a z
 // chunk) packed as problem | tile x << 16 | tile y << 32 | chunk << 48; one

@@ -132,6 +132,11 @@ template <class R>
 int run_step_adjoint(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStream_t s);
 template <class R>
 int run_step_record(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<R>* out, cudaStream_t s);
+// The parts of a record that the fused step does not make: the ratios of the
+// first pass from its recorded input field and pseudo-velocities, and, once for
+// any number of records, the density reciprocals the reverse kernels read.
+int run_record_ratios(const Prob<float>& P, const AdjPlan<float>& A, cudaStream_t s);
+int run_record_reciprocals(const Prob<float>& P, const AdjPlan<float>& A, cudaStream_t s);
 template <class R>
 int run_step_reverse(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStream_t s);
 template <class R>

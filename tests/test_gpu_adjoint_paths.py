@@ -50,3 +50,19 @@ def test_density_step_interior_warps(M, oracle, ibc):
     lam = RA.cotangents(n, sh, 19)
     for a, b in zip(RA.gpu_rho_adjoint(M, n, ibc, f, lam), RA.oracle_rho_adjoint(oracle, n, ibc, f, lam)):
         assert RA.rel(a, b) <= 1e-12
+
+
+@pytest.mark.parametrize("n,ibc,nsteps,interval", [((12, 10, 8), (0, 0, 0), 5, 2), ((70, 13, 5), (1, 1, 1), 4, 0),
+                                                   ((65, 14, 4), (1, 1, 0), 3, 3), ((9, 25, 3), (0, 1, 1), 3, 2)])
+def test_fp32_run_records_by_the_fused_kernels(M, n, ibc, nsteps, interval):
+    """A run whose interval is above one records its steps by the fused kernels,
+    the last segment's as the forward sweep passes it: psi_N has a plain run's
+    bits, and the gradients are those of an interval of one, which records by
+    the stage kernels (the same records; sums in another order, 1e-5)."""
+    f, target = A.problem(n, ibc, seed=23)
+    J, xN, gx, *gu, peak = A.gpu_adjoint_run(M, f, target, nsteps, interval=interval, precision=32)
+    J1, xN1, gx1, *gu1, _ = A.gpu_adjoint_run(M, f, target, nsteps, interval=1, precision=32)
+    np.testing.assert_array_equal(xN, xN1)
+    assert J == J1 and peak > 0
+    for a, b in zip((gx, *gu[:3]), (gx1, *gu1[:3])):
+        assert A.rel(a.astype(np.float64), b.astype(np.float64)) <= 1e-5
