@@ -179,6 +179,7 @@ __device__ __forceinline__ bool is_one(float v) { return v == 1.0f; }
 // at the rate of its five fields; six atomics a cell took 61.
 template <class R>
 __global__ void KA_LB_UPDATE ka_update(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -267,6 +268,7 @@ __device__ __forceinline__ void ka_limit_cell(const Prob<R>& P, const AdjArr<R>&
 }
 template <class R, bool NONOS>
 __global__ void KA_LB_LIMIT ka_limit(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
 #define C(IN) ka_limit_cell<R, NONOS, IN>(P, A, i, j, k)
   ADISPATCH(C)
 #undef C
@@ -410,6 +412,7 @@ __device__ __forceinline__ void ka_bounds_cell(const Prob<R>& P, const AdjArr<R>
 // 128x128x64: 25 us, 37 before.
 template <class R, bool FIRST, bool STD>
 __global__ void KA_LB_BOUNDS ka_bounds(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   __shared__ int list[128];
   __shared__ int count;
   const Geo& g = P.g;
@@ -604,6 +607,7 @@ __device__ __forceinline__ void ka_pseudo_cell(const Prob<R>& P, const AdjArr<R>
 }
 template <class R, bool AIN>
 __global__ void KA_LB_PSEUDO ka_pseudo(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -749,12 +753,14 @@ __device__ __forceinline__ void ka_cross_cell(const Prob<R>& P, const AdjArr<R>&
 }
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
 #define C(IN) ka_cross_cell<R, AIN, IN>(P, A, i, j, k)
   ADISPATCH(C)
 #undef C
 }
 template <class R>
 __global__ void __launch_bounds__(128) ka_cross_sum(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   ACELL
   const int im = wrapi(i - 1, g.np), ip = wrapi(i + 1, g.np), jm = wrapi(j - 1, g.mp), jp = wrapi(j + 1, g.mp),
             km = wrapi(k - 1, g.lp), kp = wrapi(k + 1, g.lp);
@@ -783,6 +789,7 @@ __device__ __forceinline__ void ka_update_std_cell(const Prob<R>& P, const AdjAr
 }
 template <class R>
 __global__ void __launch_bounds__(128) ka_update_std(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
 #define C(IN) ka_update_std_cell<R, IN>(P, A, i, j, k)
   ADISPATCH(C)
 #undef C
@@ -829,6 +836,7 @@ __device__ __forceinline__ void ka_limit_std_cell(const Prob<R>& P, const AdjArr
 }
 template <class R, bool NONOS>
 __global__ void __launch_bounds__(128) ka_limit_std(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
 #define C(IN) ka_limit_std_cell<R, NONOS, IN>(P, A, i, j, k)
   ADISPATCH(C)
 #undef C
@@ -969,6 +977,7 @@ __device__ __forceinline__ void ka_pseudo_std_cell(const Prob<R>& P, const AdjAr
 }
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128) ka_pseudo_std(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
 #define C(IN) ka_pseudo_std_cell<R, AIN, IN>(P, A, i, j, k)
   ADISPATCH(C)
 #undef C
@@ -1064,6 +1073,7 @@ __device__ __forceinline__ void ka_upwind_cell(const Prob<R>& P, const AdjArr<R>
 }
 template <class R, bool MF = false>
 __global__ void KA_LB_UPWIND ka_upwind(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -1089,6 +1099,7 @@ __global__ void KA_LB_UPWIND ka_upwind(const Prob<R> P, const AdjArr<R> A) {
 // that flux's adjoint through the same read maps.
 template <class R>
 __global__ void __launch_bounds__(128) ka_mass_to_w(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
   ACELL
   fx_add<R, false>(g, A.lw1, i, j, k, A.lm1.ld(i, j, k));
   fy_add<R, false>(g, A.lw2, i, j, k, A.lm2.ld(i, j, k));
@@ -1107,6 +1118,7 @@ template <class R>
 __global__ void __launch_bounds__(128) ka_rho_out(const Prob<R> P, const Arr<R> out, const Arr<R> lxc,
                                                   const Arr<R> lp1, const Arr<R> lp2, const Arr<R> lrh, Arr<R> lam,
                                                   Arr<R> g_xinc, Arr<R> g_pexe) {
+  chain_begin();
   ACELL
   (void)g;
   const R h = P.h.ld(i, j, k);
@@ -1123,6 +1135,7 @@ __global__ void __launch_bounds__(128) ka_rho_out(const Prob<R> P, const Arr<R> 
 // J's seed: lambda = psi_N - target on the interior, 0 on the halo.
 template <class R>
 __global__ void __launch_bounds__(128) ka_seed(const Prob<R> P, const Arr<R> psi, const Arr<R> target, Arr<R> lam) {
+  chain_begin();
   ACELL
   lam.at(i, j, k) = psi.ld(i, j, k) - target.ld(i, j, k);
 }
@@ -1158,12 +1171,14 @@ __global__ void __launch_bounds__(128) ka_seed(const Prob<R> P, const Arr<R> psi
   }
 template <class R>
 __global__ void __launch_bounds__(128, (KfMinBlocks<R, 8, 10>::v)) kf_upwind(const Prob<R> P) {
+  chain_begin();
 #define B(IN, U) upwind_body<R, true, false, IN, U>(P, i, j, k)
   FCELL_U(B)
 #undef B
 }
 template <class R, bool AIN, bool PV>
 __global__ void __launch_bounds__(128) kf_pairs(const Prob<R> P) {
+  chain_begin();
   ACELL
   (void)g;
   pairs_body<R, AIN, PV>(P, i, j, k);
@@ -1176,6 +1191,7 @@ struct KfPseudoMinBlocks {
 };
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128, KfPseudoMinBlocks<R>::v) kf_pseudo(const Prob<R> P) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -1222,6 +1238,7 @@ __global__ void __launch_bounds__(128, KfPseudoMinBlocks<R>::v) kf_pseudo(const 
 // recomputes its quotients from the recorded extrema and fluxes.
 template <class R, bool NONOS, bool FIRST, bool KEEP>
 __global__ void __launch_bounds__(128, (KfMinBlocks<R, 12, 12>::v)) kf_bounds(const Prob<R> P) {
+  chain_begin();
   if constexpr (NONOS && sizeof(R) == 8) {  // FP32: per-lane quotients are cheaper than the barriers
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -1246,12 +1263,14 @@ __global__ void __launch_bounds__(128, (KfMinBlocks<R, 12, 12>::v)) kf_bounds(co
 }
 template <class R, bool NONOS>
 __global__ void __launch_bounds__(128, (KfMinBlocks<R, 16, 16>::v)) kf_limit(const Prob<R> P) {
+  chain_begin();
 #define B(IN) limit_body<R, NONOS, IN>(P, i, j, k)
   FCELL(B)
 #undef B
 }
 template <class R>
 __global__ void __launch_bounds__(128) kf_update(const Prob<R> P) {
+  chain_begin();
 #define B(IN, U) update_body<R, false, IN, U>(P, i, j, k)
   FCELL_U(B)
 #undef B
@@ -1313,7 +1332,7 @@ int record_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<R>
   int n = 0;
   Prob<R> F = P;
   F.xant = A.x[0];
-  kf_upwind<R><<<grd, blk, 0, s>>>(F);
+  chain_launch(kf_upwind<R>, grd, blk, 0, s, F);
   n++;
   for (int t = 0; t < np_; t++) {
     Prob<R> Qa = pass_prob(P, A, t, true);
@@ -1326,22 +1345,22 @@ int record_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<R>
       Qa.f2 = P.f2;
       Qa.f3 = P.f3;
       if (keep_pairs) pairs_in_lf(&Qa, A);
-      if (t == 0) kf_pairs<R, true, true><<<grd, blk, 0, s>>>(Qa);
-      else kf_pairs<R, false, true><<<grd, blk, 0, s>>>(Qa);
+      if (t == 0) chain_launch(kf_pairs<R, true, true>, grd, blk, 0, s, Qa);
+      else chain_launch(kf_pairs<R, false, true>, grd, blk, 0, s, Qa);
       n++;
     }
-    if (t == 0) kf_pseudo<R, true><<<grd, blk, 0, s>>>(Qa);
-    else kf_pseudo<R, false><<<grd, blk, 0, s>>>(Qa);
+    if (t == 0) chain_launch(kf_pseudo<R, true>, grd, blk, 0, s, Qa);
+    else chain_launch(kf_pseudo<R, false>, grd, blk, 0, s, Qa);
     const Prob<R> Q = pass_prob(P, A, t, false);
     if (nonos && keep && t > 0) {  // the running extrema continue from the previous pass
       if (cudaMemcpyAsync(A.mx[t].p, A.mx[t - 1].p, ncell * sizeof(R), cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
           cudaMemcpyAsync(A.mn[t].p, A.mn[t - 1].p, ncell * sizeof(R), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
         return -5;
     }
-    if (!nonos) kf_bounds<R, false, true, false><<<grd, blk, 0, s>>>(Q);
-    else if (!keep) kf_bounds<R, true, true, false><<<grd, blk, 0, s>>>(Q);
-    else if (t == 0) kf_bounds<R, true, true, true><<<grd, blk, 0, s>>>(Q);
-    else kf_bounds<R, true, false, true><<<grd, blk, 0, s>>>(Q);
+    if (!nonos) chain_launch(kf_bounds<R, false, true, false>, grd, blk, 0, s, Q);
+    else if (!keep) chain_launch(kf_bounds<R, true, true, false>, grd, blk, 0, s, Q);
+    else if (t == 0) chain_launch(kf_bounds<R, true, true, true>, grd, blk, 0, s, Q);
+    else chain_launch(kf_bounds<R, true, false, true>, grd, blk, 0, s, Q);
     n += 2;
     // only the update and the next pass read the limited velocities: the last
     // pass of a step whose output is not wanted leaves them out
@@ -1352,11 +1371,11 @@ int record_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, const Arr<R>
     L.f1 = P.f1;
     L.f2 = P.f2;
     L.f3 = P.f3;
-    if (nonos) kf_limit<R, true><<<grd, blk, 0, s>>>(L);
-    else kf_limit<R, false><<<grd, blk, 0, s>>>(L);
+    if (nonos) chain_launch(kf_limit<R, true>, grd, blk, 0, s, L);
+    else chain_launch(kf_limit<R, false>, grd, blk, 0, s, L);
     Prob<R> U = L;
     U.xant = t < np_ - 1 ? A.x[t + 1] : *out;
-    kf_update<R><<<grd, blk, 0, s>>>(U);
+    chain_launch(kf_update<R>, grd, blk, 0, s, U);
     n += 2;
   }
   add_launches(n);
@@ -1367,7 +1386,7 @@ int run_record_ratios(const Prob<float>& P, const AdjPlan<float>& A, cudaStream_
   const Geo& g = P.g;
   const dim3 blk(32, 4, 1);
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
-  kf_bounds<float, true, true, false><<<grd, blk, 0, s>>>(pass_prob(P, A, 0, false));
+  chain_launch(kf_bounds<float, true, true, false>, grd, blk, 0, s, pass_prob(P, A, 0, false));
   add_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -1377,7 +1396,7 @@ int run_record_reciprocals(const Prob<float>& P, const AdjPlan<float>& A, cudaSt
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
   Prob<float> F = P;
   F.xant = A.x[0];  // the upwind field comes with them
-  kf_upwind<float><<<grd, blk, 0, s>>>(F);
+  chain_launch(kf_upwind<float>, grd, blk, 0, s, F);
   add_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -1420,7 +1439,7 @@ int reverse_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, bool kept, 
     m.lm1 = A.lm1;
     m.lm2 = A.lm2;
     m.lm3 = A.lm3;
-    ka_mass_to_w<R><<<grd, blk, 0, s>>>(P, m);
+    chain_launch(ka_mass_to_w<R>, grd, blk, 0, s, P, m);
     n++;
   }
   // ---- reverse, last pass first
@@ -1462,30 +1481,30 @@ int reverse_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, bool kept, 
     AdjArr<R> au = a;
     if (t < np_ - 1) au.lx.p = nullptr;
     if (P.stdf) {
-      ka_update_std<R><<<grd, blk, 0, s>>>(Q, au);
+      chain_launch(ka_update_std<R>, grd, blk, 0, s, Q, au);
       if (nonos) {
-        ka_limit_std<R, true><<<grd, blk, 0, s>>>(Q, a);
-        if (t == 0) ka_bounds<R, true, true><<<grd, blk, 0, s>>>(Q, a);
-        else ka_bounds<R, false, true><<<grd, blk, 0, s>>>(Q, a);
+        chain_launch(ka_limit_std<R, true>, grd, blk, 0, s, Q, a);
+        if (t == 0) chain_launch(ka_bounds<R, true, true>, grd, blk, 0, s, Q, a);
+        else chain_launch(ka_bounds<R, false, true>, grd, blk, 0, s, Q, a);
         n++;
       } else {
-        ka_limit_std<R, false><<<grd, blk, 0, s>>>(Q, a);
+        chain_launch(ka_limit_std<R, false>, grd, blk, 0, s, Q, a);
       }
-      if (t == 0) ka_pseudo_std<R, true><<<grd, blk, 0, s>>>(Q, a);
-      else ka_pseudo_std<R, false><<<grd, blk, 0, s>>>(Q, a);
+      if (t == 0) chain_launch(ka_pseudo_std<R, true>, grd, blk, 0, s, Q, a);
+      else chain_launch(ka_pseudo_std<R, false>, grd, blk, 0, s, Q, a);
     } else {
       if (t == np_ - 1) {  // nothing carried back, nothing added to lambda_w
         a.lmx.p = a.lmn.p = nullptr;
         if (!mass) a.lw1.p = a.lw2.p = a.lw3.p = nullptr;
       }
-      ka_update<R><<<grd, blk, 0, s>>>(Q, au);
+      chain_launch(ka_update<R>, grd, blk, 0, s, Q, au);
       if (nonos) {
-        ka_limit<R, true><<<grd, blk, 0, s>>>(Q, a);
-        if (t == 0) ka_bounds<R, true, false><<<grd, blk, 0, s>>>(Q, a);
-        else ka_bounds<R, false, false><<<grd, blk, 0, s>>>(Q, a);
+        chain_launch(ka_limit<R, true>, grd, blk, 0, s, Q, a);
+        if (t == 0) chain_launch(ka_bounds<R, true, false>, grd, blk, 0, s, Q, a);
+        else chain_launch(ka_bounds<R, false, false>, grd, blk, 0, s, Q, a);
         n++;
       } else {
-        ka_limit<R, false><<<grd, blk, 0, s>>>(Q, a);
+        chain_launch(ka_limit<R, false>, grd, blk, 0, s, Q, a);
       }
       // the pass's cp/cn/q records are dead once the reverse bounds ran:
       // they take the pair sums of its input field, and the workspace's
@@ -1497,21 +1516,21 @@ int reverse_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, bool kept, 
         Qp.f2 = P.f2;
         Qp.f3 = P.f3;
         if (kept) pairs_in_lf(&Qp, A);
-        else if (t == 0) kf_pairs<R, true, true><<<grd, blk, 0, s>>>(Qp);
-        else kf_pairs<R, false, true><<<grd, blk, 0, s>>>(Qp);
+        else if (t == 0) chain_launch(kf_pairs<R, true, true>, grd, blk, 0, s, Qp);
+        else chain_launch(kf_pairs<R, false, true>, grd, blk, 0, s, Qp);
         n += kept ? 0 : 1;
       }
       if (sizeof(R) == 4 && g.bx && g.by && g.bz) {
         if constexpr (sizeof(R) == 4) {
-          if (t == 0) ka_cross<R, true><<<grd, blk, 0, s>>>(Qp, a);
-          else ka_cross<R, false><<<grd, blk, 0, s>>>(Qp, a);
-          ka_cross_sum<R><<<grd, blk, 0, s>>>(Qp, a);
+          if (t == 0) chain_launch(ka_cross<R, true>, grd, blk, 0, s, Qp, a);
+          else chain_launch(ka_cross<R, false>, grd, blk, 0, s, Qp, a);
+          chain_launch(ka_cross_sum<R>, grd, blk, 0, s, Qp, a);
           n++;
         }
       } else if (t == 0) {
-        ka_pseudo<R, true><<<grd, blk, 0, s>>>(Qp, a);
+        chain_launch(ka_pseudo<R, true>, grd, blk, 0, s, Qp, a);
       } else {
-        ka_pseudo<R, false><<<grd, blk, 0, s>>>(Qp, a);
+        chain_launch(ka_pseudo<R, false>, grd, blk, 0, s, Qp, a);
       }
     }
     n += 3;
@@ -1526,9 +1545,9 @@ int reverse_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, bool kept, 
     a0.lm1 = A.lm1;
     a0.lm2 = A.lm2;
     a0.lm3 = A.lm3;
-    ka_upwind<R, true><<<grd, blk, 0, s>>>(P, a0);
+    chain_launch(ka_upwind<R, true>, grd, blk, 0, s, P, a0);
   } else {
-    ka_upwind<R><<<grd, blk, 0, s>>>(P, a0);
+    chain_launch(ka_upwind<R>, grd, blk, 0, s, P, a0);
   }
   n++;
   add_launches(n);
@@ -1556,7 +1575,7 @@ int run_rho_out_adjoint(const Prob<R>& P, const Arr<R>& out, const Arr<R>& lxc, 
   const Geo& g = P.g;
   const dim3 blk(32, 4, 1);
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
-  ka_rho_out<R><<<grd, blk, 0, s>>>(P, out, lxc, lp1, lp2, lrh, lam, g_xinc, g_pexe);
+  chain_launch(ka_rho_out<R>, grd, blk, 0, s, P, out, lxc, lp1, lp2, lrh, lam, g_xinc, g_pexe);
   add_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -1566,7 +1585,7 @@ int run_seed(const Prob<R>& P, const Arr<R>& psi, const Arr<R>& target, const Ar
   const Geo& g = P.g;
   const dim3 blk(32, 4, 1);
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
-  ka_seed<R><<<grd, blk, 0, s>>>(P, psi, target, lam);
+  chain_launch(ka_seed<R>, grd, blk, 0, s, P, psi, target, lam);
   add_launches(1);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

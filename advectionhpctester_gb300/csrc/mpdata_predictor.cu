@@ -71,6 +71,7 @@ __device__ __forceinline__ bool warp_unit_h(bool live, const Arr<R>& h, int i, i
 template <class R, bool R1>
 __global__ void __launch_bounds__(128) k_pred_level(Geo g, long lev, R* ox, R* oy, R* oz, Arr<R> h,
                                                     GcK<R> gc, R r) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -120,6 +121,7 @@ template <class R, bool ROLL>
 __global__ void __launch_bounds__(128) k_pred_cgrid(Geo g, long lev, R* ox, R* oy, R* oz, R* pu, R* pv,
                                                     R* pw, Arr<R> h, Arr<R> u1, Arr<R> u2, Arr<R> u3,
                                                     R r) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -213,6 +215,7 @@ int num_sms() {
 template <class R>
 __global__ void __launch_bounds__(256, 6) k_pred_cgrid_z(Geo g, long lev, R* ox, R* oy, R* oz, Arr<R> h, Arr<R> u1,
                                                       Arr<R> u2, Arr<R> u3, int kchunk) {
+  chain_begin();
   const int i = blockIdx.x * 32 + threadIdx.x + 1;
   const int j = blockIdx.y * 8 + threadIdx.y + 1;
   const int kb = blockIdx.z * kchunk + 1;
@@ -266,6 +269,7 @@ __global__ void __launch_bounds__(256, 6) k_pred_cgrid_z(Geo g, long lev, R* ox,
 template <class R, bool R1>
 __global__ void __launch_bounds__(128) k_pred_level_roll(Geo g, long lev, R* ox, R* oy, R* oz, R* pu, R* pv,
                                                          R* pw, Arr<R> h, GcK<R> gc, R r) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -285,6 +289,7 @@ __global__ void __launch_bounds__(128) k_pred_level_roll(Geo g, long lev, R* ox,
 template <class R>
 __global__ void __launch_bounds__(128) k_pred_roll(Geo g, long lev, R* ox, R* oy, R* oz, R* pu, R* pv, R* pw,
                                                    Arr<R> h, R r) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
@@ -437,24 +442,24 @@ int run_pred_parts(const PredPlan<R>& P, bool level, bool cgrid, bool roll, cuda
     if (P.prof) P.prof->begin(ST_PRED_LEVEL, s);
     const GcK<R> gc = gc_factors(P.gc1, P.gc2, P.gc3);
     if (P.dt_ratio == R(1))
-      k_pred_level<R, true><<<g1, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.h, gc, P.dt_ratio);
+      chain_launch(k_pred_level<R, true>, g1, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.h, gc, P.dt_ratio);
     else
-      k_pred_level<R, false><<<g1, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.h, gc, P.dt_ratio);
+      chain_launch(k_pred_level<R, false>, g1, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.h, gc, P.dt_ratio);
     if (P.prof) P.prof->end(ST_PRED_LEVEL, s);
     n++;
   }
   if (cgrid) {
     if (P.prof) P.prof->begin(ST_PRED_CGRID, s);
     if (roll)
-      k_pred_cgrid<R, true><<<g2, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
+      chain_launch(k_pred_cgrid<R, true>, g2, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
                                                P.dt_ratio);
     else
-      k_pred_cgrid<R, false><<<g2, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
+      chain_launch(k_pred_cgrid<R, false>, g2, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
                                                 P.dt_ratio);
     if (P.prof) P.prof->end(ST_PRED_CGRID, s);
     n++;
   } else if (roll) {
-    k_pred_roll<R><<<g1, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.dt_ratio);
+    chain_launch(k_pred_roll<R>, g1, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.dt_ratio);
     n++;
   }
   add_launches(n);
@@ -472,10 +477,10 @@ int run_predictor(const PredPlan<R>& P, cudaStream_t s) {
   const GcK<R> gc = gc_factors(P.gc1, P.gc2, P.gc3);
   if (P.prof) P.prof->begin(ST_PRED_LEVEL, s);
   if (P.dt_ratio == R(1))
-    k_pred_level_roll<R, true><<<g1, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, gc,
+    chain_launch(k_pred_level_roll<R, true>, g1, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, gc,
                                                  P.dt_ratio);
   else
-    k_pred_level_roll<R, false><<<g1, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, gc,
+    chain_launch(k_pred_level_roll<R, false>, g1, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, gc,
                                                   P.dt_ratio);
   if (P.prof) P.prof->end(ST_PRED_LEVEL, s);
   if (P.prof) P.prof->begin(ST_PRED_CGRID, s);
@@ -487,10 +492,10 @@ int run_predictor(const PredPlan<R>& P, cudaStream_t s) {
     nch = nch < 1 ? 1 : (nch > g.lp ? g.lp : nch);
     const int kchunk = (g.lp + nch - 1) / nch;
     const dim3 grid(gx, gy, (g.lp + kchunk - 1) / kchunk);
-    k_pred_cgrid_z<R><<<grid, dim3(32, 8, 1), 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.h, P.u1, P.u2, P.u3, kchunk);
+    chain_launch(k_pred_cgrid_z<R>, grid, dim3(32, 8, 1), 0, s, g, P.lev, P.ox, P.oy, P.oz, P.h, P.u1, P.u2, P.u3, kchunk);
   } else {
     // FP64: the per-cell kernel (0.272 against the z-march's 0.301 ms)
-    k_pred_cgrid<R, false><<<g2, blk, 0, s>>>(g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
+    chain_launch(k_pred_cgrid<R, false>, g2, blk, 0, s, g, P.lev, P.ox, P.oy, P.oz, P.u, P.v, P.w, P.h, P.u1, P.u2, P.u3,
                                               P.dt_ratio);
   }
   if (P.prof) P.prof->end(ST_PRED_CGRID, s);

@@ -79,12 +79,14 @@ struct MinBlocks {
 
 template <class R, bool ANTIDIFF>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_UPWIND_F64, MPDATA_MINB_UPWIND_F32>::v)) k_upwind(const Prob<R> P) {
+  chain_begin();
 #define B(IN, U) upwind_body<R, ANTIDIFF, true, IN, U>(P, i, j, k)
   CELL_DISPATCH_U(B)
 #undef B
 }
 template <class R>
 __global__ void __launch_bounds__(128) k_copy(const Prob<R> P) {
+  chain_begin();
   CELL_INDEX
   copy_body<R>(P, i, j, k);
 }
@@ -123,6 +125,7 @@ struct PseudoDefer {
 
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128, PseudoMinBlocks<R>::v) k_pseudo(const Prob<R> P) {
+  chain_begin();
   constexpr bool D = PseudoDefer<R>::v;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -164,11 +167,13 @@ __global__ void __launch_bounds__(128, PseudoMinBlocks<R>::v) k_pseudo(const Pro
 
 template <class R, bool AIN, bool PV, bool STD>
 __global__ void __launch_bounds__(128) k_pairs(const Prob<R> P) {
+  chain_begin();
   CELL_INDEX
   pairs_body<R, AIN, PV, STD>(P, i, j, k);
 }
 template <class R, bool NONOS, bool FIRST, bool KEEP>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_BOUNDS_F64, MPDATA_MINB_BOUNDS_F32>::v)) k_bounds(const Prob<R> P) {
+  chain_begin();
   if constexpr (NONOS && sizeof(R) == 8) {  // FP32: per-lane quotients are cheaper than the barriers
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -193,12 +198,14 @@ __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_BOUNDS_F64, MPD
 }
 template <class R, bool NONOS>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_LIMIT_F64, MPDATA_MINB_LIMIT_F32>::v)) k_limit(const Prob<R> P) {
+  chain_begin();
 #define B(IN) limit_body<R, NONOS, IN>(P, i, j, k)
   CELL_DISPATCH(B)
 #undef B
 }
 template <class R, bool LAST>
 __global__ void __launch_bounds__(128) k_update(const Prob<R> P) {
+  chain_begin();
 #define B(IN, U) update_body<R, LAST, IN, U>(P, i, j, k)
   CELL_DISPATCH_U(B)
 #undef B
@@ -206,6 +213,7 @@ __global__ void __launch_bounds__(128) k_update(const Prob<R> P) {
 
 template <class R, bool LINER>
 __global__ void __launch_bounds__(128) k_rho_out(const Prob<R> P) {
+  chain_begin();
   CELL_INDEX
   rho_out_body<R, LINER>(P, i, j, k);
 }
@@ -230,12 +238,12 @@ int run_step(const Prob<R>& P, int iord, int nonos, Prof* prof, cudaStream_t s) 
   const dim3 blk(32, 4, 1);
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
   if (iord < 2) {
-    LAUNCH(ST_UPWIND, (k_upwind<R, false><<<grd, blk, 0, s>>>(P)));
-    if (P.rho) LAUNCH(ST_RHO_OUT, (k_rho_out<R, true><<<grd, blk, 0, s>>>(P)));
-    else LAUNCH(ST_COPY, (k_copy<R><<<grd, blk, 0, s>>>(P)));
+    LAUNCH(ST_UPWIND, (chain_launch(k_upwind<R, false>, grd, blk, 0, s, P)));
+    if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch(k_rho_out<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_COPY, (chain_launch(k_copy<R>, grd, blk, 0, s, P)));
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
-  LAUNCH(ST_UPWIND, (k_upwind<R, true><<<grd, blk, 0, s>>>(P)));
+  LAUNCH(ST_UPWIND, (chain_launch(k_upwind<R, true>, grd, blk, 0, s, P)));
   const bool keep = iord > 2;
   // FP64: the pseudo-velocity stage reads precomputed pair sums of xant (pairs 1)
   // and, where three fields are free for them, of the pass velocities too (pairs
@@ -247,24 +255,24 @@ int run_step(const Prob<R>& P, int iord, int nonos, Prof* prof, cudaStream_t s) 
     const bool first = (pass == 2), last = (pass == iord);
     if constexpr (sizeof(R) == 8) {
       Q.pairs = P.rho || (P.stdf && !first) ? 1 : 2;
-      if (P.stdf && first) LAUNCH(ST_PAIRS, (k_pairs<R, true, true, true><<<grd, blk, 0, s>>>(Q)));
-      else if (P.stdf) LAUNCH(ST_PAIRS, (k_pairs<R, false, false, true><<<grd, blk, 0, s>>>(Q)));
-      else if (P.rho) LAUNCH(ST_PAIRS, (k_pairs<R, true, false, false><<<grd, blk, 0, s>>>(Q)));
-      else if (first) LAUNCH(ST_PAIRS, (k_pairs<R, true, true, false><<<grd, blk, 0, s>>>(Q)));
-      else LAUNCH(ST_PAIRS, (k_pairs<R, false, true, false><<<grd, blk, 0, s>>>(Q)));
+      if (P.stdf && first) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, true, true>, grd, blk, 0, s, Q)));
+      else if (P.stdf) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, false, false, true>, grd, blk, 0, s, Q)));
+      else if (P.rho) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, false, false>, grd, blk, 0, s, Q)));
+      else if (first) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, true, false>, grd, blk, 0, s, Q)));
+      else LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, false, true, false>, grd, blk, 0, s, Q)));
     }
-    if (first) LAUNCH(ST_PSEUDO, (k_pseudo<R, true><<<grd, blk, 0, s>>>(Q)));
-    else LAUNCH(ST_PSEUDO, (k_pseudo<R, false><<<grd, blk, 0, s>>>(Q)));
-    if (!nonos) LAUNCH(ST_BOUNDS, (k_bounds<R, false, true, false><<<grd, blk, 0, s>>>(P)));
-    else if (first && keep) LAUNCH(ST_BOUNDS, (k_bounds<R, true, true, true><<<grd, blk, 0, s>>>(P)));
-    else if (first) LAUNCH(ST_BOUNDS, (k_bounds<R, true, true, false><<<grd, blk, 0, s>>>(P)));
-    else LAUNCH(ST_BOUNDS, (k_bounds<R, true, false, true><<<grd, blk, 0, s>>>(P)));
-    if (nonos) LAUNCH(ST_LIMIT, (k_limit<R, true><<<grd, blk, 0, s>>>(P)));
-    else LAUNCH(ST_LIMIT, (k_limit<R, false><<<grd, blk, 0, s>>>(P)));
-    if (last) LAUNCH(ST_UPDATE, (k_update<R, true><<<grd, blk, 0, s>>>(P)));
-    else LAUNCH(ST_UPDATE, (k_update<R, false><<<grd, blk, 0, s>>>(P)));
+    if (first) LAUNCH(ST_PSEUDO, (chain_launch(k_pseudo<R, true>, grd, blk, 0, s, Q)));
+    else LAUNCH(ST_PSEUDO, (chain_launch(k_pseudo<R, false>, grd, blk, 0, s, Q)));
+    if (!nonos) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, false, true, false>, grd, blk, 0, s, P)));
+    else if (first && keep) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, true, true>, grd, blk, 0, s, P)));
+    else if (first) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, true, false>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, false, true>, grd, blk, 0, s, P)));
+    if (nonos) LAUNCH(ST_LIMIT, (chain_launch(k_limit<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_LIMIT, (chain_launch(k_limit<R, false>, grd, blk, 0, s, P)));
+    if (last) LAUNCH(ST_UPDATE, (chain_launch(k_update<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_UPDATE, (chain_launch(k_update<R, false>, grd, blk, 0, s, P)));
   }
-  if (P.rho) LAUNCH(ST_RHO_OUT, (k_rho_out<R, false><<<grd, blk, 0, s>>>(P)));
+  if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch(k_rho_out<R, false>, grd, blk, 0, s, P)));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
