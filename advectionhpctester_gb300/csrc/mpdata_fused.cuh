@@ -65,7 +65,7 @@ struct FusedArena {
 FusedArena fused_arena(const Geo& g);
 // An arena field's interior as an array view.
 Arr<float> fused_view(float* arena, int field, const Geo& g);
-// Encodes the arena's tensor map (box 72 x 20 x 1 x 1).  0 on success.
+// Encodes the arena's tensor map (box 72 x 16 x 1 x 1).  0 on success.
 int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g, int fields = FZ_NF);
 // Planes per block of the z-march for each of the n grids that one launch
 // covers (MPDATA_FUSED_KCHUNK overrides).
