@@ -171,6 +171,22 @@ __device__ __forceinline__ bool is_one(float v) { return v == 1.0f; }
   if (i > P.g.np || j > P.g.mp) return;                      \
   const Geo& g = P.g;
 
+// The workspace's fields have one layout: a cell is one offset in all of them.
+template <class R>
+struct Nbr {  // offset of a cell and differences to its neighbours, wrapped
+  long o;
+  int xm, xp, ym, yp;
+  long zm, zp;
+  __device__ __forceinline__ Nbr(const Geo& g, const Arr<R>& A, int i, int j, int k) {
+    o = A.off(i, j, k);
+    xm = i > 1 ? -1 : g.np - 1;
+    xp = i < g.np ? 1 : 1 - g.np;
+    ym = j > 1 ? -A.sy : (g.mp - 1) * A.sy;
+    yp = j < g.mp ? A.sy : (1 - g.mp) * A.sy;
+    zm = k > 1 ? -(long)A.sz : (long)(g.lp - 1) * A.sz;
+    zp = k < g.lp ? (long)A.sz : (long)(1 - g.lp) * A.sz;
+  }
+};
 // ---- update: x_new = rhr*(q - D/h), D = sum of signed limited fluxes -------
 // The adjoint of D is one value per cell (lq); the limiter's reverse takes a
 // face's lambda_w from the two cells it separates, so nothing is scattered.
@@ -226,52 +242,40 @@ __device__ __forceinline__ void min3_adj(R a, R b, R lam, const Arr<R>& La, int 
 // holds what the next pass (or the density step's mass fluxes) added to
 // lambda_w.  lambda_v is stored whole (the bounds' reverse adds to it); only
 // the ratios that limit their flux, a minority, are added to by atomics.
-template <class R, bool NONOS, bool IN>
-__device__ __forceinline__ void ka_limit_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
-  const Geo& g = P.g;
-  const R cpc = NONOS ? P.cp.ld(i, j, k) : R(0), cnc = NONOS ? P.cn.ld(i, j, k) : R(0);
-  const R lqc = A.lq.ld(i, j, k);
-#define LIMIT_FACE(V, LV, LW, IM, JM, KM, LQL, LQR)                                        \
-  {                                                                                        \
-    const R v = V.ld(i, j, k);                                                             \
-    R lw = (LQL) - (LQR);                                                                  \
-    if (LW.p) lw += LW.ld(i, j, k);                                                        \
-    if (!NONOS) {                                                                          \
-      LV.at(i, j, k) = lw;                                                                 \
-    } else {                                                                               \
-      const R cpm = P.cp.ld(IM, JM, KM), cnm = P.cn.ld(IM, JM, KM);                        \
-      /* dw/dv = a1 (v > 0), a2 (v < 0), 0; dw/da1 = pp(v), dw/da2 = -pn(v): */          \
-      /* one of them is v, the other zero */                                              \
-      const bool vz = !nonzero(v), vn = sgn(v);                                             \
-      const R a = vn ? cpm : cpc, b = vn ? cnc : cnm;                                       \
-      LV.at(i, j, k) = vz ? R(0) : lw * min3(a, b);                                         \
-      const bool tb = min3_takes_b(a, b), ta = !tb && !lt_nonneg(R(1), a);                  \
-      if (!vz && (ta || tb)) {                                                              \
-        const R m = lw * v;                                                                 \
-        const bool lower = vn == ta; /* cp is the donor-side operand a, cn is b */          \
-        atomicAdd(ta ? (lower ? &A.lcp.at(IM, JM, KM) : &A.lcp.at(i, j, k))                 \
-                     : (lower ? &A.lcn.at(IM, JM, KM) : &A.lcn.at(i, j, k)),                \
-                  m);                                                                       \
-      }                                                                                     \
-    }                                                                                       \
-  }
-  const int im = IN ? i - 1 : wrapi(i - 1, g.np), jm = IN ? j - 1 : wrapi(j - 1, g.mp), km = IN ? k - 1 : wrapi(k - 1, g.lp);
-  if (IN || g.bx || i > 1) LIMIT_FACE(P.v1, A.lv1, A.lw1, im, j, k, A.lq.ld(im, j, k), lqc)
-  if (IN || g.by || j > 1) LIMIT_FACE(P.v2, A.lv2, A.lw2, i, jm, k, A.lq.ld(i, jm, k), lqc)
-  if (IN || g.bz || k > 1) {
-    R ql = A.lq.ld(i, j, km), qr = lqc;
-    if (!g.bz && k == 2) ql = scale_up<1>(ql);
-    if (!g.bz && k == g.lp) qr = scale_up<1>(qr);
-    LIMIT_FACE(P.v3, A.lv3, A.lw3, i, j, km, ql, qr)
-  }
-#undef LIMIT_FACE
-}
 template <class R, bool NONOS>
 __global__ void KA_LB_LIMIT ka_limit(const Prob<R> P, const AdjArr<R> A) {
   chain_begin();
-#define C(IN) ka_limit_cell<R, NONOS, IN>(P, A, i, j, k)
-  ADISPATCH(C)
-#undef C
+  ACELL
+  const Nbr<R> n(g, A.lq, i, j, k);
+  const long o = n.o, ov = P.v1.off(i, j, k);  // the recorded velocities may lie in a padded arena
+  const R *const cp = P.cp.p + o, *const cn = P.cn.p + o, *const lq = A.lq.p + o;
+  const R cpc = NONOS ? cp[0] : R(0), cnc = NONOS ? cn[0] : R(0), qc = lq[0];
+  auto face = [&](const Arr<R>& V, const Arr<R>& LV, const Arr<R>& LW, long d, R ql, R qr) {
+    const R v = V.p[ov];
+    R lw = ql - qr;
+    if (LW.p) lw += LW.p[o];
+    if (!NONOS) {
+      LV.p[o] = lw;
+      return;
+    }
+    // dw/dv = a1 (v > 0), a2 (v < 0), 0; dw/da1 = pp(v), dw/da2 = -pn(v): one of
+    // them is v, the other zero.  cp is of the cell the flux enters, cn of the
+    // one it leaves
+    const R cpm = cp[d], cnm = cn[d];
+    const bool vz = !nonzero(v), vn = sgn(v);
+    const R a = vn ? cpm : cpc, b = vn ? cnc : cnm;
+    LV.p[o] = vz ? R(0) : lw * min3(a, b);
+    const bool tb = min3_takes_b(a, b), ta = !tb && !lt_nonneg(R(1), a);
+    if (!vz && (ta || tb)) atomicAdd((ta ? A.lcp.p : A.lcn.p) + (vn == ta ? o + d : o), lw * v);
+  };
+  if (g.bx || i > 1) face(P.v1, A.lv1, A.lw1, n.xm, lq[n.xm], qc);
+  if (g.by || j > 1) face(P.v2, A.lv2, A.lw2, n.ym, lq[n.ym], qc);
+  if (g.bz || k > 1) {
+    R ql = lq[n.zm], qr = qc;
+    if (!g.bz && k == 2) ql = scale_up<1>(ql);
+    if (!g.bz && k == g.lp) qr = scale_up<1>(qr);
+    face(P.v3, A.lv3, A.lw3, n.zm, ql, qr);
+  }
 }
 
 // ---- bounds: cp = (mx-x)h/Dp, cn = (x-mn)h/Dn -------------------------------
@@ -664,27 +668,33 @@ __global__ void KA_LB_PSEUDO ka_pseudo(const Prob<R> P, const AdjArr<R> A) {
 // lower faces themselves, a second one adds the shifted sums.  The pair sums
 // and velocity pairs come from kf_pairs, the six fields from the standard
 // form's accumulators.
-// 128x128x64: 44 + 14 us, 89 by scatter.
-template <class R, bool AIN, bool IN>
-__device__ __forceinline__ void ka_cross_cell(const Prob<R>& P, const AdjArr<R>& A, int i, int j, int k) {
-  const Geo& g = P.g;
+// Both kernels are bound by issue and load latency: the workspace's fields have
+// one layout, so a cell is one offset in all of them and a neighbour one
+// difference, instead of index arithmetic per load (850 instructions a cell
+// before).  128x128x64: 27 + 11 us (44 + 14 with it), 89 by scatter.
+template <class R, bool AIN>
+__global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R> A) {
+  chain_begin();
+  ACELL
+  const Nbr<R> n(g, P.cp, i, j, k);
+  const long o = n.o;
   const Arr<R>& U1 = AIN ? P.u1 : P.w1;
   const Arr<R>& U2 = AIN ? P.u2 : P.w2;
   const Arr<R>& U3 = AIN ? P.u3 : P.w3;
-  const int im = IN ? i - 1 : wrapi(i - 1, g.np), ip = IN ? i + 1 : wrapi(i + 1, g.np);
-  const int jm = IN ? j - 1 : wrapi(j - 1, g.mp), jp = IN ? j + 1 : wrapi(j + 1, g.mp);
-  const int km = IN ? k - 1 : wrapi(k - 1, g.lp), kp = IN ? k + 1 : wrapi(k + 1, g.lp);
-  const R x = P.xant.ld(i, j, k);
-  const R f1 = P.f1.ld(i, j, k), f2 = P.f2.ld(i, j, k), f3 = P.f3.ld(i, j, k);
-  R lx, C1, C2, C3, T1, T2, T3;
-  auto face = [&](const Arr<R>& LV, const Arr<R>& U, const Arr<R>& HM, int a, int b, int c, R xl, R xr_, R cr4) {
-    return FaceAdj<R, false>(LV.ld(a, b, c), U.ld(a, b, c), HM.ld(a, b, c), xl, xr_, cr4);
-  };
-  {  // x: cross differences along y and z
-    const R S2 = P.f2.ld(im, j, k) + f2, S3 = P.f3.ld(im, j, k) + f3;
-    const R D2 = P.cp.ld(i, jp, k) - P.cp.ld(i, jm, k), D3 = P.cp.ld(i, j, kp) - P.cp.ld(i, j, km);
-    const FaceAdj<R, false> f = face(A.lv1, U1, P.hmx, i, j, k, P.xant.ld(im, j, k), x, S2 * D2 + S3 * D3);
-    A.la1.at(i, j, k) += f.la;
+  const R* const u1 = U1.p + U1.off(i, j, k);
+  const R* const u2 = U2.p + U2.off(i, j, k);
+  const R* const u3 = U3.p + U3.off(i, j, k);
+  const R* const X = P.xant.p + P.xant.off(i, j, k);
+  const R *const cp = P.cp.p + o, *const cn = P.cn.p + o, *const q = P.q.p + o;
+  const R *const F1 = P.f1.p + o, *const F2 = P.f2.p + o, *const F3 = P.f3.p + o;
+  const R *const lv1 = A.lv1.p + o, *const lv2 = A.lv2.p + o, *const lv3 = A.lv3.p + o;
+  const R *const hx = P.hmx.p + o, *const hy = P.hmy.p + o, *const hz = P.hmz.p + o;
+  const R x = X[0], f1 = F1[0], f2 = F2[0], f3 = F3[0];
+  R lx, C1, C2, C3, T1, T2, T3, la1, la2, la3;
+  {  // x: cross differences along y and z; the lower face, then the upper one
+    const R S2 = F2[n.xm] + f2, S3 = F3[n.xm] + f3, D2 = cp[n.yp] - cp[n.ym], D3 = cp[n.zp] - cp[n.zm];
+    const FaceAdj<R, false> f(lv1[0], u1[0], hx[0], X[n.xm], x, S2 * D2 + S3 * D3);
+    la1 = f.la;
     C2 = f.lcr4 * D2;
     T2 = f.lcr4 * S2;
     C3 = f.lcr4 * D3;
@@ -692,9 +702,9 @@ __device__ __forceinline__ void ka_cross_cell(const Prob<R>& P, const AdjArr<R>&
     lx = f.lK;
   }
   {
-    const R S2 = f2 + P.f2.ld(ip, j, k), S3 = f3 + P.f3.ld(ip, j, k);
-    const R D2 = P.cp.ld(ip, jp, k) - P.cp.ld(ip, jm, k), D3 = P.cp.ld(ip, j, kp) - P.cp.ld(ip, j, km);
-    const FaceAdj<R, false> f = face(A.lv1, U1, P.hmx, ip, j, k, x, x, R(0));
+    const R S2 = f2 + F2[n.xp], S3 = f3 + F3[n.xp], D2 = cp[n.xp + n.yp] - cp[n.xp + n.ym],
+            D3 = cp[n.xp + n.zp] - cp[n.xp + n.zm];
+    const FaceAdj<R, false> f(lv1[n.xp], u1[n.xp], hx[n.xp], x, x, R(0));
     C2 += f.lcr4 * D2;
     T2 += f.lcr4 * S2;
     C3 += f.lcr4 * D3;
@@ -702,73 +712,70 @@ __device__ __forceinline__ void ka_cross_cell(const Prob<R>& P, const AdjArr<R>&
     lx -= f.lK;
   }
   {  // y: along x and z
-    const R S1 = P.f1.ld(i, jm, k) + f1, S3 = P.f3.ld(i, jm, k) + f3;
-    const R D1 = P.cn.ld(ip, j, k) - P.cn.ld(im, j, k), D3 = P.cn.ld(i, j, kp) - P.cn.ld(i, j, km);
-    const FaceAdj<R, false> f = face(A.lv2, U2, P.hmy, i, j, k, P.xant.ld(i, jm, k), x, S1 * D1 + S3 * D3);
-    A.la2.at(i, j, k) += f.la;
+    const int ux = (j < g.mp ? 1 : 1 - g.mp) * U2.sy;
+    const R S1 = F1[n.ym] + f1, S3 = F3[n.ym] + f3, D1 = cn[n.xp] - cn[n.xm], D3 = cn[n.zp] - cn[n.zm];
+    const FaceAdj<R, false> f(lv2[0], u2[0], hy[0], X[(j > 1 ? -1 : g.mp - 1) * P.xant.sy], x, S1 * D1 + S3 * D3);
+    la2 = f.la;
     C1 = f.lcr4 * D1;
     T1 = f.lcr4 * S1;
     C3 += f.lcr4 * D3;
     T3 += f.lcr4 * S3;
     lx += f.lK;
-  }
-  {
-    const R S1 = f1 + P.f1.ld(i, jp, k), S3 = f3 + P.f3.ld(i, jp, k);
-    const R D1 = P.cn.ld(ip, jp, k) - P.cn.ld(im, jp, k), D3 = P.cn.ld(i, jp, kp) - P.cn.ld(i, jp, km);
-    const FaceAdj<R, false> f = face(A.lv2, U2, P.hmy, i, jp, k, x, x, R(0));
-    C1 += f.lcr4 * D1;
-    T1 += f.lcr4 * S1;
-    C3 += f.lcr4 * D3;
-    T3 += f.lcr4 * S3;
-    lx -= f.lK;
+    const R S1p = f1 + F1[n.yp], S3p = f3 + F3[n.yp], D1p = cn[n.yp + n.xp] - cn[n.yp + n.xm],
+            D3p = cn[n.yp + n.zp] - cn[n.yp + n.zm];
+    const FaceAdj<R, false> p(lv2[n.yp], u2[ux], hy[n.yp], x, x, R(0));
+    C1 += p.lcr4 * D1p;
+    T1 += p.lcr4 * S1p;
+    C3 += p.lcr4 * D3p;
+    T3 += p.lcr4 * S3p;
+    lx -= p.lK;
   }
   {  // z: along x and y
-    const R S1 = P.f1.ld(i, j, km) + f1, S2 = P.f2.ld(i, j, km) + f2;
-    const R D1 = P.q.ld(ip, j, k) - P.q.ld(im, j, k), D2 = P.q.ld(i, jp, k) - P.q.ld(i, jm, k);
-    const FaceAdj<R, false> f = face(A.lv3, U3, P.hmz, i, j, k, P.xant.ld(i, j, km), x, S1 * D1 + S2 * D2);
-    A.la3.at(i, j, k) += f.la;
+    const long ux = (long)(k < g.lp ? 1 : 1 - g.lp) * U3.sz, xz = (long)(k > 1 ? -1 : g.lp - 1) * P.xant.sz;
+    const R S1 = F1[n.zm] + f1, S2 = F2[n.zm] + f2, D1 = q[n.xp] - q[n.xm], D2 = q[n.yp] - q[n.ym];
+    const FaceAdj<R, false> f(lv3[0], u3[0], hz[0], X[xz], x, S1 * D1 + S2 * D2);
+    la3 = f.la;
     C1 += f.lcr4 * D1;
     T1 += f.lcr4 * S1;
     C2 += f.lcr4 * D2;
     T2 += f.lcr4 * S2;
     lx += f.lK;
+    const R S1p = f1 + F1[n.zp], S2p = f2 + F2[n.zp], D1p = q[n.zp + n.xp] - q[n.zp + n.xm],
+            D2p = q[n.zp + n.yp] - q[n.zp + n.ym];
+    const FaceAdj<R, false> p(lv3[n.zp], u3[ux], hz[n.zp], x, x, R(0));
+    C1 += p.lcr4 * D1p;
+    T1 += p.lcr4 * S1p;
+    C2 += p.lcr4 * D2p;
+    T2 += p.lcr4 * S2p;
+    lx -= p.lK;
   }
-  {
-    const R S1 = f1 + P.f1.ld(i, j, kp), S2 = f2 + P.f2.ld(i, j, kp);
-    const R D1 = P.q.ld(ip, j, kp) - P.q.ld(im, j, kp), D2 = P.q.ld(i, jp, kp) - P.q.ld(i, jm, kp);
-    const FaceAdj<R, false> f = face(A.lv3, U3, P.hmz, i, j, kp, x, x, R(0));
-    C1 += f.lcr4 * D1;
-    T1 += f.lcr4 * S1;
-    C2 += f.lcr4 * D2;
-    T2 += f.lcr4 * S2;
-    lx -= f.lK;
-  }
-  A.lxant.at(i, j, k) += lx;
-  A.lg1.at(i, j, k) = C1;
-  A.lg2.at(i, j, k) = C2;
-  A.lg3.at(i, j, k) = C3;
-  A.lf1.at(i, j, k) = T1;
-  A.lf2.at(i, j, k) = T2;
-  A.lf3.at(i, j, k) = T3;
-}
-template <class R, bool AIN>
-__global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R> A) {
-  chain_begin();
-#define C(IN) ka_cross_cell<R, AIN, IN>(P, A, i, j, k)
-  ADISPATCH(C)
-#undef C
+  const R l0 = A.lxant.p[o], a1 = A.la1.ld(i, j, k), a2 = A.la2.ld(i, j, k), a3 = A.la3.ld(i, j, k);
+  A.lxant.p[o] = l0 + lx;
+  A.la1.at(i, j, k) = a1 + la1;
+  A.la2.at(i, j, k) = a2 + la2;
+  A.la3.at(i, j, k) = a3 + la3;
+  A.lg1.p[o] = C1;
+  A.lg2.p[o] = C2;
+  A.lg3.p[o] = C3;
+  A.lf1.p[o] = T1;
+  A.lf2.p[o] = T2;
+  A.lf3.p[o] = T3;
 }
 template <class R>
 __global__ void __launch_bounds__(128) ka_cross_sum(const Prob<R> P, const AdjArr<R> A) {
   chain_begin();
   ACELL
-  const int im = wrapi(i - 1, g.np), ip = wrapi(i + 1, g.np), jm = wrapi(j - 1, g.mp), jp = wrapi(j + 1, g.mp),
-            km = wrapi(k - 1, g.lp), kp = wrapi(k + 1, g.lp);
-  A.lxant.at(i, j, k) += (A.lf1.ld(im, j, k) - A.lf1.ld(ip, j, k)) + (A.lf2.ld(i, jm, k) - A.lf2.ld(i, jp, k)) +
-                         (A.lf3.ld(i, j, km) - A.lf3.ld(i, j, kp));
-  A.la1.at(i, j, k) += A.lg1.ld(im, j, k) + A.lg1.ld(i, j, k);
-  A.la2.at(i, j, k) += A.lg2.ld(i, jm, k) + A.lg2.ld(i, j, k);
-  A.la3.at(i, j, k) += A.lg3.ld(i, j, km) + A.lg3.ld(i, j, k);
+  const Nbr<R> n(g, A.lg1, i, j, k);
+  const long o = n.o;
+  const R *const g1 = A.lg1.p + o, *const g2 = A.lg2.p + o, *const g3 = A.lg3.p + o;
+  const R *const t1 = A.lf1.p + o, *const t2 = A.lf2.p + o, *const t3 = A.lf3.p + o;
+  const R lx = A.lxant.p[o] + ((t1[n.xm] - t1[n.xp]) + (t2[n.ym] - t2[n.yp]) + (t3[n.zm] - t3[n.zp]));
+  const R a1 = A.la1.ld(i, j, k) + (g1[n.xm] + g1[0]), a2 = A.la2.ld(i, j, k) + (g2[n.ym] + g2[0]),
+          a3 = A.la3.ld(i, j, k) + (g3[n.zm] + g3[0]);
+  A.lxant.p[o] = lx;
+  A.la1.at(i, j, k) = a1;
+  A.la2.at(i, j, k) = a2;
+  A.la3.at(i, j, k) = a3;
 }
 
 // ---- standard form (antidiff3d-standard-gpubc.f90) ---------------------------
