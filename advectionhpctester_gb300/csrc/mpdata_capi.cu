@@ -1287,7 +1287,6 @@ int adj_plan(Workspace* w, Prob<R>* P, AdjPlan<R>* A, const R* psi_in, const R* 
   for (int c = 0; c < 3; c++) A->lf[c] = next();
   A->lq = next();
   A->pass_acc_elems = 12 * n;
-  A->lxin = next();
   A->acc_elems = (size_t)(a + f * n - A->acc);
   A->lam = caller_view<R>(lambda, ih, sx, sy);
   A->gu1 = caller_view<R>(gu1, ih, sx + 1, sy);

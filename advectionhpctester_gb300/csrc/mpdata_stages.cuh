@@ -110,8 +110,8 @@ struct AdjPlan {
   Arr<R> lx[kAdjMaxPass], lw[kAdjMaxPass][3], lmx[kAdjMaxPass], lmn[kAdjMaxPass];
   Arr<R> lv[3], lcp, lcn;                       // reused by every pass
   Arr<R> lg[3], lf[3], lq;                      // reused by every pass (standard form)
-  Arr<R> lxin;                                  // adjoint of the step's input psi
   Arr<R> lam;                                   // caller lambda: in dJ/dpsi_new, out dJ/dpsi_in
+                                                // (the accumulator once the last pass's update has read it)
   Arr<R> gu1, gu2, gu3;                         // caller gradients of u1..u3
   R* acc;                                       // the accumulators, contiguous
   size_t acc_elems, pass_acc_elems;             // all of them; the per-pass block (lv, lcp, lcn)
@@ -125,8 +125,8 @@ struct AdjPlan {
 // Fields of the arena for iord passes: records, then accumulators.
 // records per pass: x, v*3, w*3, cp, cn, mx, mn, fns*3, q
 inline size_t adj_record_fields(int iord) { return (size_t)(iord - 1) * 15; }
-// accumulators: per pass lx, lw*3, lmx, lmn; shared lv*3, lcp, lcn, lg*3, lf*3, lq; lxin
-inline size_t adj_acc_fields(int iord) { return (size_t)(iord - 1) * 6 + 12 + 1; }
+// accumulators: per pass lx, lw*3, lmx, lmn; shared lv*3, lcp, lcn, lg*3, lf*3, lq
+inline size_t adj_acc_fields(int iord) { return (size_t)(iord - 1) * 6 + 12; }
 
 template <class R>
 int run_step_adjoint(const Prob<R>& P, const AdjPlan<R>& A, int nonos, cudaStream_t s);
