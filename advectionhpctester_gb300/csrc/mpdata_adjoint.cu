@@ -671,7 +671,7 @@ __global__ void KA_LB_PSEUDO ka_pseudo(const Prob<R> P, const AdjArr<R> A) {
 // Both kernels are bound by issue and load latency: the workspace's fields have
 // one layout, so a cell is one offset in all of them and a neighbour one
 // difference, instead of index arithmetic per load (850 instructions a cell
-// before).  128x128x64: 27 + 11 us (44 + 14 with it), 89 by scatter.
+// before).  128x128x64: 28 + 13 us (44 + 14 with it), 89 by scatter.
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R> A) {
   chain_begin();
@@ -749,11 +749,10 @@ __global__ void __launch_bounds__(128) ka_cross(const Prob<R> P, const AdjArr<R>
     T2 += p.lcr4 * S2p;
     lx -= p.lK;
   }
-  const R l0 = A.lxant.p[o], a1 = A.la1.ld(i, j, k), a2 = A.la2.ld(i, j, k), a3 = A.la3.ld(i, j, k);
-  A.lxant.p[o] = l0 + lx;
-  A.la1.at(i, j, k) = a1 + la1;
-  A.la2.at(i, j, k) = a2 + la2;
-  A.la3.at(i, j, k) = a3 + la3;
+  A.lxant.p[o] += lx;
+  addat(A.la1, i, j, k, la1);  // the caller's gradients: steps on other streams may add to them
+  addat(A.la2, i, j, k, la2);
+  addat(A.la3, i, j, k, la3);
   A.lg1.p[o] = C1;
   A.lg2.p[o] = C2;
   A.lg3.p[o] = C3;
@@ -770,12 +769,10 @@ __global__ void __launch_bounds__(128) ka_cross_sum(const Prob<R> P, const AdjAr
   const R *const g1 = A.lg1.p + o, *const g2 = A.lg2.p + o, *const g3 = A.lg3.p + o;
   const R *const t1 = A.lf1.p + o, *const t2 = A.lf2.p + o, *const t3 = A.lf3.p + o;
   const R lx = A.lxant.p[o] + ((t1[n.xm] - t1[n.xp]) + (t2[n.ym] - t2[n.yp]) + (t3[n.zm] - t3[n.zp]));
-  const R a1 = A.la1.ld(i, j, k) + (g1[n.xm] + g1[0]), a2 = A.la2.ld(i, j, k) + (g2[n.ym] + g2[0]),
-          a3 = A.la3.ld(i, j, k) + (g3[n.zm] + g3[0]);
   A.lxant.p[o] = lx;
-  A.la1.at(i, j, k) = a1;
-  A.la2.at(i, j, k) = a2;
-  A.la3.at(i, j, k) = a3;
+  addat(A.la1, i, j, k, g1[n.xm] + g1[0]);
+  addat(A.la2, i, j, k, g2[n.ym] + g2[0]);
+  addat(A.la3, i, j, k, g3[n.zm] + g3[0]);
 }
 
 // ---- standard form (antidiff3d-standard-gpubc.f90) ---------------------------
@@ -996,9 +993,10 @@ __global__ void __launch_bounds__(128) ka_pseudo_std(const Prob<R> P, const AdjA
 //
 // A cell owns its lower face on each axis (the last cell of an open axis the
 // upper one as well) and forms that face's lambda_F from both of its cells:
-// three fluxes a cell instead of six, one atomic each (the donor cell's), the
-// velocity gradient by a plain read and write.  256x256x64 FP64: 142 us, half
-// of it the FP64 pipe's; six fluxes from a cell and a copy of the result 167.
+// three fluxes a cell instead of six, one atomic each to the donor cell and to the
+// velocity gradient (steps on other streams may add to the same gradients).
+// 256x256x64 FP64: 116 us (142 with a plain read and write of the gradients);
+// six fluxes from a cell and a copy of the result 167.
 // MF (density step): the step also outputs each face's upwind flux as part
 // of its mass flux: the lower face's flux of every cell (u1(i), u2(j), u3(k))
 // and the upper face's of the last cell along each axis (u1(np+1), ...),
@@ -1014,7 +1012,7 @@ __device__ __forceinline__ void flux_adj(R lF, R u, R xl, R xr_, R* GU, const Ar
   } else {
     if (l_var) addat(Lx, li, lj, lk, m);
   }
-  if (nonzero(u)) *GU += lF * (sgn(u) ? xr_ : xl);
+  if (nonzero(u)) atomicAdd(GU, lF * (sgn(u) ? xr_ : xl));
 }
 
 // U: rhr and hinv are exactly 1 at the cells read (x*1 == x); an instantiation,

@@ -66,3 +66,39 @@ def test_fp32_run_records_by_the_fused_kernels(M, n, ibc, nsteps, interval):
     assert J == J1 and peak > 0
     for a, b in zip((gx, *gu[:3]), (gx1, *gu1[:3])):
         assert A.rel(a.astype(np.float64), b.astype(np.float64)) <= 1e-5
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_two_streams_add_to_the_same_gradients(M, precision):
+    """Step adjoints on two streams add their dJ/du into one set of arrays: the
+    sum of both, whatever the interleaving (rounding of two sums, 1e-5 and 1e-13)."""
+    import torch
+    dt = np.float32 if precision == 32 else np.float64
+    f, _ = A.problem((96, 40, 16), (1, 1, 1), seed=3)
+    rng = np.random.default_rng(4)
+    d = {k: M.fortran_device(getattr(f, k), dtype=dt) for k in ("x", "u1", "u2", "u3", "h", "rhr", "bcx", "bcy")}
+    lams = [np.asfortranarray(rng.uniform(-1, 1, f.x.shape)) for _ in range(2)]
+    ws = [M.Workspace(f.np, f.mp, f.lp, f.ih, 1, 1, 1, iord=2, nonos=1, gauge=1, precision=precision) for _ in range(2)]
+    zeros = lambda: [torch.zeros_like(d[k]) for k in ("u1", "u2", "u3")]
+
+    def add(w, lam, gu, stream=None):
+        l = M.fortran_device(lam, dtype=dt)
+        torch.cuda.synchronize()
+        for _ in range(8):
+            l2 = l.clone()
+            torch.cuda.current_stream().synchronize()
+            w.step_adjoint(d["x"], d["u1"], d["u2"], d["u3"], d["h"], d["rhr"], l2, *gu, d["bcx"], d["bcy"], stream=stream)
+            yield l2
+
+    want = zeros()
+    for w, lam in zip(ws, lams):
+        keep = list(add(w, lam, want))
+    torch.cuda.synchronize()
+    got, streams = zeros(), [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    keep = list(zip(add(ws[0], lams[0], got, streams[0].cuda_stream), add(ws[1], lams[1], got, streams[1].cuda_stream)))
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        assert A.rel(M.to_numpy(a).astype(np.float64), M.to_numpy(b).astype(np.float64)) <= (1e-5 if precision == 32 else 1e-13)
+    for w in ws:
+        w.close()
