@@ -904,7 +904,13 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
     rc = check_grid(&g);
     if (rc) { delete b; return rc; }
     b->ncell[p] = (size_t)q.np * q.mp * q.lp;
-    if (fused_eligible(geo_of(g), precision, q.gauge, nonos, iord, 0)) b->fzi[p] = b->nfz++;
+    if (fused_eligible(geo_of(g), precision, q.gauge, nonos, iord, 0)) {
+      // a work item holds 16 bits of the tile's x index: 64-cell tiles; walled and
+      // standard-form rows keep the limit of the tile kernels' 32-cell ones
+      const int tile = fused_class(geo_of(g), q.gauge) == FZ_PERIODIC ? 64 : 32;
+      if ((q.np + tile - 1) / tile > 65536) { delete b; return MPDATA_E_DIMS; }
+      b->fzi[p] = b->nfz++;
+    }
     // a velocity group is shared within the fused problems or within the others
     int own = p;
     for (int r = 0; r < p; r++)
