@@ -911,11 +911,14 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       if ((q.np + tile - 1) / tile > 65536) { delete b; return MPDATA_E_DIMS; }
       b->fzi[p] = b->nfz++;
     }
-    // a velocity group is shared within the fused problems or within the others
+    // a velocity group is shared within the fused periodic gauge problems or within
+    // the others
+    auto apart = [&](int r) {
+      return b->fzi[r] >= 0 && probs[r].gauge && probs[r].ibcx && probs[r].ibcy && probs[r].ibcz;
+    };
     int own = p;
     for (int r = 0; r < p; r++)
-      if (probs[r].velocity_group == q.velocity_group && b->owner[r] == r &&
-          (b->fzi[r] >= 0) == (b->fzi[p] >= 0)) { own = r; break; }
+      if (probs[r].velocity_group == q.velocity_group && b->owner[r] == r && apart(r) == apart(p)) { own = r; break; }
     if (own != p) {  // sharing a velocity needs the same grid and boundaries
       const mpdata_problem& o2 = probs[own];
       if (o2.np != q.np || o2.mp != q.mp || o2.lp != q.lp || o2.ibcx != q.ibcx || o2.ibcy != q.ibcy ||

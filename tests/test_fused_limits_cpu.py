@@ -1,6 +1,7 @@
 """Size limits of the fused FP32 kernels, checked before a call touches the GPU:
 the 16-bit tile index of a batch's work items, and the 32-bit plane strides of
-the fused arena, whose halo is wider than the caller's."""
+the fused arena, whose halo is wider than the caller's; and which problems of a
+velocity group are held to one grid."""
 import ctypes
 
 import pytest
@@ -28,12 +29,21 @@ def test_batch_refuses_rows_beyond_the_tile_index(native_lib, ibc, gauge, most):
     assert create(native_lib, [(most, 2, 2, *ibc, gauge, 0)]) != E_DIMS
 
 
+@pytest.mark.parametrize("a,b,refused", [
+    ((8, 8, 8, 1, 1, 1, 1, 0), (9, 8, 8, 1, 1, 1, 1, 0), True),    # two fields on one velocity
+    ((8, 8, 8, 0, 0, 0, 1, 0), (9, 8, 8, 0, 0, 0, 0, 0), True),
+    ((8, 8, 8, 1, 1, 1, 1, 0), (9, 8, 8, 1, 1, 1, 0, 0), False),   # periodic gauge fields keep their own
+    ((8, 8, 8, 0, 0, 0, 1, 0), (8, 8, 8, 1, 1, 1, 1, 0), False)])
+def test_velocity_group_of_periodic_gauge_and_other_problems(native_lib, a, b, refused):
+    assert (create(native_lib, [a, b]) == E_DIMS) == refused
+
+
 class Geo(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in ("np", "mp", "lp", "ih", "bx", "by", "bz")]
 
 
-@pytest.mark.parametrize("np_,mp,fits", [(512, 512, True), (300000000, 2, True), (357913932, 2, True), (357913933, 2, False),
-                                         (400000000, 2, False)])
+@pytest.mark.parametrize("np_,mp,fits", [(512, 512, True), (300000000, 2, True), (357913932, 2, True),
+                                         (357913933, 2, False), (400000000, 2, False)])
 def test_arena_planes_stay_below_32_bit_strides(native_lib, np_, mp, fits):
     """Grids whose own planes have 32-bit strides but whose arena planes (rows
     of np+8, mp+4 rows) do not keep the stage kernels."""
