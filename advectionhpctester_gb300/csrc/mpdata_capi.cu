@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -96,9 +97,10 @@ struct Workspace {
   cudaStream_t last;
   EventProf* prof;
   void* adj;  // adjoint scratch (10 fields), allocated on first use
-  // fused single-precision path (periodic gauge grids): its arena shares
-  // `mem` with the stage path's scratch, which it never needs at the same time
-  bool fused;
+  // fused single-precision path: its arena shares `mem` with the stage path's
+  // scratch, which it never needs at the same time
+  FusedClass cls;  // the step's kernels
+  bool fz_records; // an adjoint run's records may be made by the fused kernels
   int fz_kchunk;
   int fz_mx, fz_mn;    // arena fields holding the last fused step's extrema (-1: none)
   bool fz_extrema;     // the last step ran fused: the extrema live in the arena
@@ -168,10 +170,11 @@ Prob<R> make_prob(const mpdata_grid& g, int gauge, R* psi, const R* u1, const R*
 }
 
 // The fused step's arguments for the problem P.
-FusedPlan fused_plan(const Prob<float>& P, float* arena, int kchunk, int* err, const CUtensorMap* map) {
+FusedPlan fused_plan(const Prob<float>& P, FusedClass cls, float* arena, int kchunk, int* err,
+                     const CUtensorMap* map) {
   FusedPlan F;
   F.g = P.g;
-  F.cls = fused_class(P.g, !P.stdf);
+  F.cls = cls;
   F.bcx = P.bcx;
   F.bcy = P.bcy;
   F.psi = P.psi;
@@ -192,8 +195,8 @@ FusedPlan fused_plan(const Prob<float>& P, float* arena, int kchunk, int* err, c
 template <class R>
 int ws_step(Workspace* w, const Prob<R>& P, Prof* prof, cudaStream_t s) {
   if constexpr (sizeof(R) == 4) {
-    if (w->fused) {
-      const FusedPlan F = fused_plan(P, static_cast<float*>(w->mem), w->fz_kchunk, w->d_err, &w->fz_map);
+    if (w->cls != FZ_NONE) {
+      const FusedPlan F = fused_plan(P, w->cls, static_cast<float*>(w->mem), w->fz_kchunk, w->d_err, &w->fz_map);
       w->fz_extrema = true;
       return run_step_fused(F, w->o.iord, prof, s, &w->fz_mx, &w->fz_mn) == 0 ? MPDATA_OK : MPDATA_E_CUDA;
     }
@@ -388,8 +391,8 @@ int count_violations(Workspace* w, const void* psi, double tol, unsigned long lo
   const Prob<R> P = make_prob<R>(w->g, w->o.gauge, x, x, x, x, x, x, nullptr, nullptr, base, w->ncell,
                                  base + (size_t)NFIELD * w->ncell, 1);
   if (w->fz_extrema && w->fz_mx >= 0) {  // the last step ran fused: its extrema are arena fields
-    const Arr<float> fx = fused_view(static_cast<float*>(w->mem), w->fz_mx, P.g),
-                     fn = fused_view(static_cast<float*>(w->mem), w->fz_mn, P.g);
+    const Arr<float> fx = fused_view(static_cast<float*>(w->mem), w->fz_mx, P.g, w->cls),
+                     fn = fused_view(static_cast<float*>(w->mem), w->fz_mn, P.g, w->cls);
     const Arr<R> mx{reinterpret_cast<R*>(fx.p), fx.sy, fx.sz}, mn{reinterpret_cast<R*>(fn.p), fn.sy, fn.sz};
     return run_bound_violations<R>(P.g, P.psi, mx, mn, tol, d, s) ? MPDATA_E_CUDA : MPDATA_OK;
   }
@@ -419,15 +422,17 @@ int mpdata_ws_create(const mpdata_grid* grid, const mpdata_opts* opts, void** ws
   w->prof = nullptr;
   w->adj = nullptr;
   w->nhi = (size_t)grid->mp * grid->lp + (size_t)grid->np * grid->lp + (size_t)grid->np * grid->mp;
-  w->fused = fused_eligible(geo_of(*grid), opts->precision, opts->gauge, opts->nonos, opts->iord, 0);
+  const Geo geo = geo_of(*grid);
+  fused_classes(&geo, &opts->gauge, 1, opts->precision, opts->nonos, opts->iord, &w->cls);
+  const char* env = std::getenv("MPDATA_FUSED");
+  w->fz_records = opts->gauge && opts->iord == 2 && !(env && env[0] == '0') &&
+                  fused_eligible(geo, opts->precision, opts->gauge, opts->nonos, opts->iord, 0);
   w->fz_mx = w->fz_mn = -1;
   w->fz_extrema = false;
   size_t elems = w->ncell * NSCRATCH + w->nhi;
-  if (w->fused) {
-    const Geo fg = geo_of(*grid);
-    fused_kchunk(&fg, 1, &w->fz_kchunk);
-    const size_t fz = fused_arena(geo_of(*grid)).elems;
-    if (fz > elems) elems = fz;
+  if (w->cls != FZ_NONE) {
+    fused_kchunk(&geo, &w->cls, 1, &w->fz_kchunk);
+    elems = std::max(elems, fused_arena(geo, w->cls).elems);
   }
   if (cudaMalloc(&w->mem, elems * w->elem) != cudaSuccess) {
     cudaGetLastError();
@@ -440,7 +445,7 @@ int mpdata_ws_create(const mpdata_grid* grid, const mpdata_opts* opts, void** ws
     delete w;
     return MPDATA_E_CUDA;
   }
-  if (w->fused && fused_make_tmap(&w->fz_map, static_cast<float*>(w->mem), geo_of(*grid))) {
+  if (w->cls != FZ_NONE && fused_make_tmap(&w->fz_map, static_cast<float*>(w->mem), geo, w->cls)) {
     cudaFree(w->mem);
     cudaFree(w->d_err);
     delete w;
@@ -679,17 +684,17 @@ struct Batch {
   cudaStream_t cap;             // private stream used only for graph capture
   EventProf* prof;
   cudaStream_t last;
-  // problems on the fused single-precision kernels (FP32 periodic gauge
-  // problems, as single steps take them): one launch per fused kernel for
-  // all of them; the others run on the tile kernels above
+  // problems on the fused single-precision kernels: one launch per fused kernel
+  // and work list for all of them; the others run on the tile kernels above
+  std::vector<FusedClass> cls;     // each problem's kernels
   std::vector<int> fzi;            // index in the fused table, or -1
   int nfz;
   std::vector<int> fz_kchunk;      // z-march chunk of each fused problem
   std::vector<FusedArgs> fz_args;  // host image of the fused table
   void* d_fz;
   void* d_maps;                    // one tensor map per fused problem
-  unsigned long long* d_items;     // work items: the periodic gauge problems', then the others'
-  FusedItems fz_items[2];
+  unsigned long long* d_items;     // work items, list after list
+  FusedItems fz_items[FZ_NLIST];
   int* d_err;
 };
 
@@ -828,21 +833,7 @@ bool write_prob(Batch* b, int p, void* psi, const void* u1, const void* u2, cons
   if constexpr (sizeof(R) == 4) {
     const int f = b->fzi[p];
     if (f >= 0) {
-      FusedPlan F;
-      F.g = P.g;
-      F.cls = fused_class(P.g, !P.stdf);
-      F.bcx = P.bcx;
-      F.bcy = P.bcy;
-      F.psi = P.psi;
-      F.u1 = P.u1;
-      F.u2 = P.u2;
-      F.u3 = P.u3;
-      F.h = P.h;
-      F.rhr = P.rhr;
-      F.arena = base + b->foff[p];
-      F.kchunk = b->fz_kchunk[f];
-      F.err = b->d_err;
-      F.tmap = nullptr;
+      const FusedPlan F = fused_plan(P, b->cls[p], base + b->foff[p], b->fz_kchunk[f], b->d_err, nullptr);
       const FusedArgs A = fused_args(F);
       changed = changed || memcmp(&b->fz_args[f], &A, sizeof A) != 0;
       b->fz_args[f] = A;
@@ -896,21 +887,32 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   b->d_items = nullptr;
   for (FusedItems& I : b->fz_items) I = FusedItems{nullptr, 0};
   b->d_err = nullptr;
-  size_t off = 0;
+  std::vector<Geo> geos(nprob);
+  std::vector<int> gauge(nprob);
   for (int p = 0; p < nprob; p++) {
     const mpdata_problem& q = probs[p];
     if (q.gauge != 0 && q.gauge != 1) { delete b; return MPDATA_E_OPTS; }
     mpdata_grid g{q.np, q.mp, q.lp, ih, q.ibcx, q.ibcy, q.ibcz};
     rc = check_grid(&g);
     if (rc) { delete b; return rc; }
-    b->ncell[p] = (size_t)q.np * q.mp * q.lp;
-    if (fused_eligible(geo_of(g), precision, q.gauge, nonos, iord, 0)) {
-      // a work item holds 16 bits of the tile's x index: 64-cell tiles; walled and
-      // standard-form rows keep the limit of the tile kernels' 32-cell ones
-      const int tile = fused_class(geo_of(g), q.gauge) == FZ_PERIODIC ? 64 : 32;
-      if ((q.np + tile - 1) / tile > 65536) { delete b; return MPDATA_E_DIMS; }
-      b->fzi[p] = b->nfz++;
+    geos[p] = geo_of(g);
+    gauge[p] = q.gauge;
+  }
+  b->cls.resize(nprob);
+  fused_classes(geos.data(), gauge.data(), nprob, precision, nonos, iord, b->cls.data());
+  size_t off = 0;
+  for (int p = 0; p < nprob; p++) {
+    const mpdata_problem& q = probs[p];
+    const mpdata_grid g = grid_of(b, p);
+    // a work item holds 16 bits of the tile's x index: 64-cell tiles; the problems
+    // that the tile kernels may take keep the limit of their 32-cell ones
+    const int tile = b->cls[p] == FZ_PERIODIC ? 64 : 32;
+    if (fused_eligible(geos[p], precision, q.gauge, nonos, iord, 0) && (q.np + tile - 1) / tile > 65536) {
+      delete b;
+      return MPDATA_E_DIMS;
     }
+    b->ncell[p] = (size_t)q.np * q.mp * q.lp;
+    if (b->cls[p] != FZ_NONE) b->fzi[p] = b->nfz++;
     // a velocity group is shared within the fused periodic gauge problems or within
     // the others
     auto apart = [&](int r) {
@@ -927,7 +929,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
     b->owner[p] = own;
     b->foff[p] = off;
     size_t nf = (size_t)NFIELD * b->ncell[p];
-    if (b->fzi[p] >= 0) nf = std::max(nf, fused_arena(geo_of(g)).elems);
+    if (b->fzi[p] >= 0) nf = std::max(nf, fused_arena(geo_of(g), b->cls[p]).elems);
     off += (nf + 63) / 64 * 64;  // 256-byte aligned regions (TMA wants 16)
   }
   // a group of two or more fields shares the velocity-only terms of its
@@ -973,23 +975,25 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   if (ok && b->nfz) {
     // fused problems: argument table, tensor maps of their arenas, work items
     std::vector<CUtensorMap> maps(b->nfz);
-    std::vector<unsigned long long> items[2], last;  // last: the lighter gauge blocks end the second list
-    std::vector<Geo> geos;
+    std::vector<unsigned long long> items[FZ_NLIST], last[FZ_NLIST], all;
+    std::vector<Geo> fg;
+    std::vector<FusedClass> fc;
     for (int p = 0; p < nprob; p++)
-      if (b->fzi[p] >= 0) geos.push_back(geo_of(grid_of(b, p)));
+      if (b->fzi[p] >= 0) {
+        fg.push_back(geos[p]);
+        fc.push_back(b->cls[p]);
+      }
     b->fz_kchunk.resize(b->nfz);
-    fused_kchunk(geos.data(), b->nfz, b->fz_kchunk.data());
-    for (int p = 0; p < nprob && ok; p++) {
-      const int f = b->fzi[p];
-      if (f < 0) continue;
-      const Geo g = geo_of(grid_of(b, p));
-      ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], g) == 0;
-      const FusedClass c = fused_class(g, probs[p].gauge);
-      fused_items(g, b->fz_kchunk[f], f, c == FZ_PERIODIC ? items[0] : c == FZ_STD ? items[1] : last);
+    fused_kchunk(fg.data(), fc.data(), b->nfz, b->fz_kchunk.data());
+    for (int f = 0, p = 0; p < nprob && ok; p++) {
+      if (b->fzi[p] < 0) continue;
+      ok = fused_make_tmap(&maps[f], static_cast<float*>(b->mem) + b->foff[p], fg[f], fc[f]) == 0;
+      // the lighter gauge blocks end the list they share with the standard form's
+      fused_items(fg[f], fc[f], b->fz_kchunk[f], f, fc[f] == FZ_WALL ? last : items);
+      f++;
     }
-    std::vector<unsigned long long> all;
-    items[1].insert(items[1].end(), last.begin(), last.end());
-    for (int c = 0; c < 2; c++) all.insert(all.end(), items[c].begin(), items[c].end());
+    items[FZ_L_MIXED].insert(items[FZ_L_MIXED].end(), last[FZ_L_MIXED].begin(), last[FZ_L_MIXED].end());
+    for (const auto& list : items) all.insert(all.end(), list.begin(), list.end());
     ok = ok && all.size() < 0x7fffffffu && fused_init() == 0 &&
          cudaMalloc(&b->d_fz, b->nfz * sizeof(FusedArgs)) == cudaSuccess &&
          cudaMalloc(&b->d_maps, b->nfz * sizeof(CUtensorMap)) == cudaSuccess &&
@@ -1000,7 +1004,7 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
          cudaMemcpy(b->d_items, all.data(), all.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice) ==
              cudaSuccess;
     size_t at = 0;
-    for (int c = 0; c < 2; c++) {
+    for (int c = 0; c < FZ_NLIST; c++) {
       b->fz_items[c] = FusedItems{b->d_items + at, (int)items[c].size()};
       at += items[c].size();
     }
@@ -1393,10 +1397,13 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
   // one record arena per step of a segment (of the stage kernels' ones the
   // workspace's own is the first)
   const size_t nrec = adj_record_fields(w->o.iord);
-  const FusedArena fa = fused_arena(P.g);
+  const FusedClass rcls = g.ibcx && g.ibcy && g.ibcz ? FZ_PERIODIC : FZ_WALL;  // the records' kernels
+  const FusedArena fa = fused_arena(P.g, rcls);
+  int rchunk = 0;
+  fused_kchunk(&P.g, &rcls, 1, &rchunk);
   const size_t fz_flags = (size_t)FZ_NREC * fa.fs, fz_tail = fz_flags + ((size_t)fa.ntx * fa.nty * P.g.lp + 3) / 4;
   const size_t fz_elems = (fz_tail + 3 * w->ncell + 63) / 64 * 64;
-  bool fz = sizeof(R) == 4 && K > 1 && w->fused && w->o.gauge && w->o.iord == 2;
+  bool fz = sizeof(R) == 4 && K > 1 && w->fz_records;
   const size_t rec_bytes = fz ? fz_elems * sizeof(R) : nrec * w->ncell * w->elem;
   const size_t nrecs = fz ? K : K - 1;
   R* recs = nullptr;
@@ -1418,9 +1425,9 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
         maps.resize((size_t)K);
         for (int k = 0; k < K && !rc; k++) {
           R* a = recs + (size_t)k * fz_elems;
-          if (fused_make_tmap(&maps[k], a, P.g, FZ_NREC)) rc = MPDATA_E_CUDA;
-          plans[k].x[0] = fused_view(a, FZ_X0, P.g);
-          for (int c = 0; c < 3; c++) plans[k].v[0][c] = fused_view(a, FZ_V1 + c, P.g);
+          if (fused_make_tmap(&maps[k], a, P.g, rcls, FZ_NREC)) rc = MPDATA_E_CUDA;
+          plans[k].x[0] = fused_view(a, FZ_X0, P.g, rcls);
+          for (int c = 0; c < 3; c++) plans[k].v[0][c] = fused_view(a, FZ_V1 + c, P.g, rcls);
           Arr<R>* const ratios[3] = {&plans[k].cp[0], &plans[k].cn[0], &plans[k].q[0]};
           for (int c = 0; c < 3; c++) *ratios[c] = scratch_view<R>(a + fz_tail + (size_t)c * w->ncell, P.g);
         }
@@ -1446,7 +1453,7 @@ int adjoint_run_impl(void* ws, int nsteps, int interval, R* psi, const R* u1, co
       Prob<R> B = P;
       B.psi = caller_view<R>(dst ? dst : src, ih, sx, sy);
       R* const a = recs + (size_t)slot * fz_elems;
-      FusedPlan F = fused_plan(B, a, w->fz_kchunk, w->d_err, &maps[slot]);
+      FusedPlan F = fused_plan(B, rcls, a, rchunk, w->d_err, &maps[slot]);
       F.flags = reinterpret_cast<unsigned char*>(a + fz_flags);
       if (dst && cudaMemcpyAsync(dst, src, pbytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return MPDATA_E_CUDA;
       if (run_record_fused(F, dst != nullptr, s)) return MPDATA_E_CUDA;

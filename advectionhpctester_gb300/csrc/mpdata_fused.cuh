@@ -1,4 +1,5 @@
-// Host interface of the fused single-precision MPDATA step (mpdata_fused.cu).
+// Host interface of the fused single-precision MPDATA step (mpdata_fused.cu,
+// mpdata_narrow.cu).
 #pragma once
 #include <cuda.h>
 
@@ -9,17 +10,18 @@
 namespace mpdata {
 
 // Fields of the fused step's arena, each px*(mp+4)*lp floats (a halo of four
-// columns and two rows on every side; rows a multiple of 4 elements so that
-// every row starts on a 16-byte boundary, as TMA requires): the step's input
-// field, the two ping-pong fields of the passes, pseudo and limited
-// velocities, and two ping-pong pairs of running extrema.
+// columns and two rows on every side, none for the narrow kernels; rows a
+// multiple of 4 elements so that every row starts on a 16-byte boundary, as TMA
+// requires): the step's input field, the two ping-pong fields of the passes,
+// pseudo and limited velocities, and two ping-pong pairs of running extrema.
 enum FusedField { FZ_XIN = 0, FZ_X0, FZ_X1, FZ_V1, FZ_V2, FZ_V3, FZ_W1, FZ_W2, FZ_W3, FZ_MX0, FZ_MN0, FZ_MX1,
                   FZ_MN1, FZ_NF };
 
-// The kernel instantiations a problem runs on: the gauge form on a grid that is
-// periodic on every axis (wraps only), the gauge form with open or wall axes,
-// the standard form on any grid.
-enum FusedClass { FZ_PERIODIC = 0, FZ_WALL, FZ_STD };
+// The kernels a problem runs on: the gauge form on a grid that is periodic on
+// every axis (wraps only) by 64x12 tiles or by narrow ones, the gauge form with
+// open or wall axes, the standard form on any grid; FZ_NONE: the stage kernels
+// (in a batch the tile kernels).
+enum FusedClass { FZ_NONE = -1, FZ_PERIODIC = 0, FZ_NARROW, FZ_WALL, FZ_STD };
 
 // Arguments of the fused kernels for one problem: caller arrays, the arena,
 // the z-march chunk, and the arena fields of the current pass.
@@ -51,25 +53,28 @@ struct FusedPlan {
   unsigned char* flags = nullptr;  // the unit flags, where they do not follow the FZ_NF fields
 };
 
-// Whether a step takes the fused path: FP32, nonoscillatory, iord >= 2, not the
-// density step.
+// Whether the fused kernels on 64x12 tiles can take a step: FP32, nonoscillatory,
+// iord >= 2, not the density step.
 bool fused_eligible(const Geo& g, int precision, int gauge, int nonos, int iord, int rho);
-FusedClass fused_class(const Geo& g, int gauge);
-// Arena geometry: row pitch, elements per field, tiles, and the total elements
-// of the FZ_NF fields and the flags.
+// The kernels of n problems that are stepped together (cls[p]).  FP32 steps with
+// the limiter and iord >= 2, outside the density step, run on the fused kernels
+// where these are the faster ones.
+void fused_classes(const Geo* g, const int* gauge, int n, int precision, int nonos, int iord, FusedClass* cls);
+// Arena geometry of a class: row pitch, elements per field, tiles, and the total
+// elements of the FZ_NF fields and the flags.
 struct FusedArena {
   int px, ntx, nty;
   long fs;
   size_t elems;
 };
-FusedArena fused_arena(const Geo& g);
+FusedArena fused_arena(const Geo& g, FusedClass c);
 // An arena field's interior as an array view.
-Arr<float> fused_view(float* arena, int field, const Geo& g);
-// Encodes the arena's tensor map (box 72 x 16 x 1 x 1).  0 on success.
-int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g, int fields = FZ_NF);
-// Planes per block of the z-march for each of the n grids that one launch
-// covers (MPDATA_FUSED_KCHUNK overrides).
-void fused_kchunk(const Geo* g, int n, int* kchunk);
+Arr<float> fused_view(float* arena, int field, const Geo& g, FusedClass c);
+// Encodes the arena's tensor map (one field's box in a plane).  0 on success.
+int fused_make_tmap(CUtensorMap* map, float* arena, const Geo& g, FusedClass c, int fields = FZ_NF);
+// Planes per block of the z-march for each of the n problems that are stepped
+// together (MPDATA_FUSED_KCHUNK overrides).
+void fused_kchunk(const Geo* g, const FusedClass* c, int n, int* kchunk);
 // One step; on return *mx_field / *mn_field name the arena fields that hold
 // the running extrema of the step (-1 when iord = 2 keeps none).
 int run_step_fused(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int* mx_field, int* mn_field);
@@ -83,10 +88,17 @@ int run_record_fused(const FusedPlan& F, bool update, cudaStream_t s);
 
 // Batches.  Each problem of the fused table gets work items (a tile and a z
 // chunk) packed as problem | tile x << 16 | tile y << 32 | chunk << 48; one
-// launch per fused kernel and work list (the periodic gauge problems; the others)
+// launch per fused kernel and work list (the periodic gauge problems; the walled
+// and standard-form ones; the narrow ones, whose first kernel has its own tiles)
 // then covers every problem.
 FusedArgs fused_args(const FusedPlan& F);
-void fused_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& items);
+enum FusedList { FZ_L_PERIODIC = 0, FZ_L_MIXED, FZ_L_NARROW_UP, FZ_L_NARROW, FZ_NLIST };
+inline unsigned long long pack_item(int p, int x, int y, int z) {
+  return (unsigned long long)p | ((unsigned long long)x << 16) | ((unsigned long long)y << 32) |
+         ((unsigned long long)z << 48);
+}
+// Appends problem p's items to its lists (items[FZ_NLIST]).
+void fused_items(const Geo& g, FusedClass c, int kchunk, int p, std::vector<unsigned long long>* items);
 int fused_init();
 // A device work list.
 struct FusedItems {
@@ -94,8 +106,19 @@ struct FusedItems {
   int n;
 };
 // One step of every problem of the table (device arrays: args, tensor maps;
-// items: the two lists, empty ones with n = 0).
+// items[FZ_NLIST]: the lists, empty ones with n = 0).
 int run_batch_fused(const FusedArgs* probs, const CUtensorMap* maps, const FusedItems* items, int iord, Prof* prof,
                     cudaStream_t s);
+
+// The narrow kernels' part of the above.
+FusedArena narrow_arena(const Geo& g);
+int narrow_make_tmap(CUtensorMap* map, float* arena, const Geo& g);
+void narrow_kchunk(const Geo* g, int n, int* kchunk);
+void narrow_items(const Geo& g, int kchunk, int p, std::vector<unsigned long long>& up,
+                  std::vector<unsigned long long>& rest);
+int narrow_init();
+int narrow_step(const FusedPlan& F, int iord, Prof* prof, cudaStream_t s, int* mx_field, int* mn_field);
+int narrow_batch(const FusedArgs* probs, const CUtensorMap* maps, const FusedItems& up, const FusedItems& rest,
+                 int iord, Prof* prof, cudaStream_t s);
 
 }  // namespace mpdata
