@@ -1,5 +1,6 @@
 """Which kernels an FP32 step takes and how many planes a block marches: a grid
-that fills the 64x12 tiles badly is not sent to them."""
+that fills the 64x12 tiles badly is not sent to them, a list of equal grids counts
+rounds of resident blocks."""
 import ctypes
 
 import pytest
@@ -68,7 +69,15 @@ def chunks(lib, sizes, cls, ibc=PER):
 
 @pytest.mark.parametrize("count,size,cls,want", [
     (1, (128, 128, 64), PERIODIC, 5), (1, (512, 512, 128), PERIODIC, 19),
+    (2, (80, 32, 32), WALL, 3),        # 47 us, 61 with the 1 plane of the rule for uneven lists
+    (6, (80, 32, 32), PERIODIC, 4),    # 56 : 76
+    (24, (48, 48, 48), STD, 16),       # 246 : 303
     (64, (32, 32, 32), NARROW, 16), (6, (32, 32, 32), NARROW, 3)])
-def test_chunk(native_lib, monkeypatch, count, size, cls, want):
+def test_equal_grids_count_rounds(native_lib, monkeypatch, count, size, cls, want):
     monkeypatch.delenv("MPDATA_FUSED_KCHUNK", raising=False)
     assert chunks(native_lib, [size] * count, [cls] * count) == [want] * count
+
+
+def test_both_forms_on_one_grid_keep_the_average(native_lib, monkeypatch):
+    monkeypatch.delenv("MPDATA_FUSED_KCHUNK", raising=False)
+    assert chunks(native_lib, [(127, 95, 48)] * 12, [STD] + [WALL] * 5 + [STD] * 6, OPEN) == [8] * 12
