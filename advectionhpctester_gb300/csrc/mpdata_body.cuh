@@ -46,6 +46,9 @@ struct Prob {
   R* f1hi;  // (mp,lp)
   R* f2hi;  // (np,lp)
   R* f3hi;  // (np,mp)
+  // the step's kernels are launched to follow one another (chain_launch_if).  Last: four
+  // bytes before the views moved the parameters' words and cost the FP32 upwind 7%
+  int chained;
 };
 
 // ---- read helpers -------------------------------------------------------

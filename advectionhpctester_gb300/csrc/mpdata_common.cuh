@@ -9,6 +9,41 @@
 
 namespace mpdata {
 
+// Launches a kernel so that it may start while the one before it in the stream
+// drains: its blocks take the slots that the last wave leaves free and wait in
+// chain_begin() until every block of that kernel is done and its writes are
+// visible.  Saves the launch latency between the short kernels of a step; a
+// launch that follows a copy, a memset or another library's kernel waits for it
+// as usual.  Every kernel launched this way calls chain_begin() before it
+// touches memory, so each one's end also implies the end of all before it.
+// chained = false: an ordinary launch, after the end of the one before.
+template <class... P, class... A>
+inline void chain_launch_if(bool chained, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                            A&&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute a;
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  chain_launch_if(true, kernel, grid, block, smem, s, std::forward<A>(args)...);
+}
+// The two halves: the following kernel may start; this one's inputs are there.
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_begin() {
+  chain_trigger();
+  chain_wait();
+}
+
 // Grid geometry and boundary flags (1 = periodic axis).
 struct Geo {
   int np, mp, lp, ih;
@@ -20,35 +55,6 @@ struct Geo {
 // allocation.  Indices are the reference's 1-based (i,j,k).  The strides are
 // 32-bit (the host rejects grids whose planes, halos included, reach 2^31
 // elements), so each term of an offset is one 32x32->64 multiply-add.
-// Launches a kernel so that it may start while the one before it in the stream
-// drains: its blocks take the slots that the last wave leaves free and wait in
-// chain_begin() until every block of that kernel is done and its writes are
-// visible.  Saves the launch latency between the short kernels of a step; a
-// launch that follows a copy, a memset or another library's kernel waits for it
-// as usual.  Every kernel launched this way calls chain_begin() before it
-// touches memory, so each one's end also implies the end of all before it.
-template <class... P, class... A>
-inline void chain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
-  cudaLaunchConfig_t c = {};
-  c.gridDim = grid;
-  c.blockDim = block;
-  c.dynamicSmemBytes = smem;
-  c.stream = s;
-  cudaLaunchAttribute a;
-  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  a.val.programmaticStreamSerializationAllowed = 1;
-  c.attrs = &a;
-  c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
-}
-// The two halves: the following kernel may start; this one's inputs are there.
-__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void chain_begin() {
-  chain_trigger();
-  chain_wait();
-}
-
 template <class R>
 struct Arr {
   R* p;

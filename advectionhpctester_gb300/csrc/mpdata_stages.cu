@@ -79,14 +79,14 @@ struct MinBlocks {
 
 template <class R, bool ANTIDIFF>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_UPWIND_F64, MPDATA_MINB_UPWIND_F32>::v)) k_upwind(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
 #define B(IN, U) upwind_body<R, ANTIDIFF, true, IN, U>(P, i, j, k)
   CELL_DISPATCH_U(B)
 #undef B
 }
 template <class R>
 __global__ void __launch_bounds__(128) k_copy(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
   CELL_INDEX
   copy_body<R>(P, i, j, k);
 }
@@ -125,7 +125,7 @@ struct PseudoDefer {
 
 template <class R, bool AIN>
 __global__ void __launch_bounds__(128, PseudoMinBlocks<R>::v) k_pseudo(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
   constexpr bool D = PseudoDefer<R>::v;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -167,13 +167,13 @@ __global__ void __launch_bounds__(128, PseudoMinBlocks<R>::v) k_pseudo(const Pro
 
 template <class R, bool AIN, bool PV, bool STD>
 __global__ void __launch_bounds__(128) k_pairs(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
   CELL_INDEX
   pairs_body<R, AIN, PV, STD>(P, i, j, k);
 }
 template <class R, bool NONOS, bool FIRST, bool KEEP>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_BOUNDS_F64, MPDATA_MINB_BOUNDS_F32>::v)) k_bounds(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
   if constexpr (NONOS && sizeof(R) == 8) {  // FP32: per-lane quotients are cheaper than the barriers
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -198,14 +198,14 @@ __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_BOUNDS_F64, MPD
 }
 template <class R, bool NONOS>
 __global__ void __launch_bounds__(128, (MinBlocks<R, MPDATA_MINB_LIMIT_F64, MPDATA_MINB_LIMIT_F32>::v)) k_limit(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
 #define B(IN) limit_body<R, NONOS, IN>(P, i, j, k)
   CELL_DISPATCH(B)
 #undef B
 }
 template <class R, bool LAST>
 __global__ void __launch_bounds__(128) k_update(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
 #define B(IN, U) update_body<R, LAST, IN, U>(P, i, j, k)
   CELL_DISPATCH_U(B)
 #undef B
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(128) k_update(const Prob<R> P) {
 
 template <class R, bool LINER>
 __global__ void __launch_bounds__(128) k_rho_out(const Prob<R> P) {
-  chain_begin();
+  if (P.chained) chain_begin();
   CELL_INDEX
   rho_out_body<R, LINER>(P, i, j, k);
 }
@@ -232,18 +232,38 @@ void add_launches(int n) { __atomic_add_fetch(&g_launches, (unsigned long long)n
     add_launches(1);                         \
   } while (0)
 
+// Whether a step's kernels follow one another without the launch gap
+// (chain_launch_if); blocks: of one kernel.  It saves two or three microseconds a
+// kernel, 10 to 30% of a small step.  It costs where long kernels are bound by memory:
+// the next one's blocks start as the last ones end, in another order over the SMs
+// and their L2 halves (FP32 upwind step on 255x193x65, 25480 blocks: 51.7 us plain,
+// 59.4 chained; 512x512x128 434 and 585; limiter off 0.87 of the chained time there;
+// 128x128x64, 8192 blocks: 1.06 to 1.11).  And where an FP64 grid has one to four
+// blocks an SM: the waiting blocks pile up on the SMs whose own end first, and the
+// FP64 pipes of the others idle (gauge step on 32^3, 256 blocks: 40.4 us plain, 48.7
+// chained; standard form 45.4 and 59.9; 33^3, 594 blocks: 47.3 and 50.0; but 24^3, 144
+// blocks: 35.9 and 32.8; 40^3, 800 blocks: 1.04 to 1.12 of the chained time).
+// The FP32 density step, whose predictor runs before it, keeps 3 to 5% of its chain.
+bool chain_pays(long blocks, bool f64, int iord, bool limited_or_std, bool rho) {
+  if (iord < 2 || !(f64 || rho)) return blocks <= 12000;
+  if (!f64) return true;
+  return !(limited_or_std && blocks >= 210 && blocks <= 700);
+}
+
 template <class R>
-int run_step(const Prob<R>& P, int iord, int nonos, Prof* prof, cudaStream_t s) {
-  const Geo& g = P.g;
+int run_step(const Prob<R>& P0, int iord, int nonos, Prof* prof, cudaStream_t s) {
+  const Geo& g = P0.g;
   const dim3 blk(32, 4, 1);
   const dim3 grd((g.np + 31) / 32, (g.mp + 3) / 4, g.lp);
+  Prob<R> P = P0;
+  P.chained = chain_pays((long)grd.x * grd.y * grd.z, sizeof(R) == 8, iord, nonos || P.stdf, P.rho);
   if (iord < 2) {
-    LAUNCH(ST_UPWIND, (chain_launch(k_upwind<R, false>, grd, blk, 0, s, P)));
-    if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch(k_rho_out<R, true>, grd, blk, 0, s, P)));
-    else LAUNCH(ST_COPY, (chain_launch(k_copy<R>, grd, blk, 0, s, P)));
+    LAUNCH(ST_UPWIND, (chain_launch_if(P.chained, k_upwind<R, false>, grd, blk, 0, s, P)));
+    if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch_if(P.chained, k_rho_out<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_COPY, (chain_launch_if(P.chained, k_copy<R>, grd, blk, 0, s, P)));
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
   }
-  LAUNCH(ST_UPWIND, (chain_launch(k_upwind<R, true>, grd, blk, 0, s, P)));
+  LAUNCH(ST_UPWIND, (chain_launch_if(P.chained, k_upwind<R, true>, grd, blk, 0, s, P)));
   const bool keep = iord > 2;
   // FP64: the pseudo-velocity stage reads precomputed pair sums of xant (pairs 1)
   // and, where three fields are free for them, of the pass velocities too (pairs
@@ -255,24 +275,24 @@ int run_step(const Prob<R>& P, int iord, int nonos, Prof* prof, cudaStream_t s) 
     const bool first = (pass == 2), last = (pass == iord);
     if constexpr (sizeof(R) == 8) {
       Q.pairs = P.rho || (P.stdf && !first) ? 1 : 2;
-      if (P.stdf && first) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, true, true>, grd, blk, 0, s, Q)));
-      else if (P.stdf) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, false, false, true>, grd, blk, 0, s, Q)));
-      else if (P.rho) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, false, false>, grd, blk, 0, s, Q)));
-      else if (first) LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, true, true, false>, grd, blk, 0, s, Q)));
-      else LAUNCH(ST_PAIRS, (chain_launch(k_pairs<R, false, true, false>, grd, blk, 0, s, Q)));
+      if (P.stdf && first) LAUNCH(ST_PAIRS, (chain_launch_if(P.chained, k_pairs<R, true, true, true>, grd, blk, 0, s, Q)));
+      else if (P.stdf) LAUNCH(ST_PAIRS, (chain_launch_if(P.chained, k_pairs<R, false, false, true>, grd, blk, 0, s, Q)));
+      else if (P.rho) LAUNCH(ST_PAIRS, (chain_launch_if(P.chained, k_pairs<R, true, false, false>, grd, blk, 0, s, Q)));
+      else if (first) LAUNCH(ST_PAIRS, (chain_launch_if(P.chained, k_pairs<R, true, true, false>, grd, blk, 0, s, Q)));
+      else LAUNCH(ST_PAIRS, (chain_launch_if(P.chained, k_pairs<R, false, true, false>, grd, blk, 0, s, Q)));
     }
-    if (first) LAUNCH(ST_PSEUDO, (chain_launch(k_pseudo<R, true>, grd, blk, 0, s, Q)));
-    else LAUNCH(ST_PSEUDO, (chain_launch(k_pseudo<R, false>, grd, blk, 0, s, Q)));
-    if (!nonos) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, false, true, false>, grd, blk, 0, s, P)));
-    else if (first && keep) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, true, true>, grd, blk, 0, s, P)));
-    else if (first) LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, true, false>, grd, blk, 0, s, P)));
-    else LAUNCH(ST_BOUNDS, (chain_launch(k_bounds<R, true, false, true>, grd, blk, 0, s, P)));
-    if (nonos) LAUNCH(ST_LIMIT, (chain_launch(k_limit<R, true>, grd, blk, 0, s, P)));
-    else LAUNCH(ST_LIMIT, (chain_launch(k_limit<R, false>, grd, blk, 0, s, P)));
-    if (last) LAUNCH(ST_UPDATE, (chain_launch(k_update<R, true>, grd, blk, 0, s, P)));
-    else LAUNCH(ST_UPDATE, (chain_launch(k_update<R, false>, grd, blk, 0, s, P)));
+    if (first) LAUNCH(ST_PSEUDO, (chain_launch_if(P.chained, k_pseudo<R, true>, grd, blk, 0, s, Q)));
+    else LAUNCH(ST_PSEUDO, (chain_launch_if(P.chained, k_pseudo<R, false>, grd, blk, 0, s, Q)));
+    if (!nonos) LAUNCH(ST_BOUNDS, (chain_launch_if(P.chained, k_bounds<R, false, true, false>, grd, blk, 0, s, P)));
+    else if (first && keep) LAUNCH(ST_BOUNDS, (chain_launch_if(P.chained, k_bounds<R, true, true, true>, grd, blk, 0, s, P)));
+    else if (first) LAUNCH(ST_BOUNDS, (chain_launch_if(P.chained, k_bounds<R, true, true, false>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_BOUNDS, (chain_launch_if(P.chained, k_bounds<R, true, false, true>, grd, blk, 0, s, P)));
+    if (nonos) LAUNCH(ST_LIMIT, (chain_launch_if(P.chained, k_limit<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_LIMIT, (chain_launch_if(P.chained, k_limit<R, false>, grd, blk, 0, s, P)));
+    if (last) LAUNCH(ST_UPDATE, (chain_launch_if(P.chained, k_update<R, true>, grd, blk, 0, s, P)));
+    else LAUNCH(ST_UPDATE, (chain_launch_if(P.chained, k_update<R, false>, grd, blk, 0, s, P)));
   }
-  if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch(k_rho_out<R, false>, grd, blk, 0, s, P)));
+  if (P.rho) LAUNCH(ST_RHO_OUT, (chain_launch_if(P.chained, k_rho_out<R, false>, grd, blk, 0, s, P)));
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
