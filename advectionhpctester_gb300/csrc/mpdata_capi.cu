@@ -904,8 +904,11 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
   for (int p = 0; p < nprob; p++) {
     const mpdata_problem& q = probs[p];
     const mpdata_grid g = grid_of(b, p);
-    // a work item holds 16 bits of the tile's x index: 64-cell tiles; the problems
-    // that the tile kernels may take keep the limit of their 32-cell ones
+    // a work item holds 16 bits of the tile's x index: 64-cell tiles (a single narrow
+    // row beyond 32-cell ones moves there); the problems that the tile kernels may take
+    // keep the limit of their 32-cell tiles
+    if (b->cls[p] == FZ_NARROW && q.np > 32 * 65536 && fused_eligible(geos[p], precision, q.gauge, nonos, iord, 0))
+      b->cls[p] = FZ_PERIODIC;
     const int tile = b->cls[p] == FZ_PERIODIC ? 64 : 32;
     if (fused_eligible(geos[p], precision, q.gauge, nonos, iord, 0) && (q.np + tile - 1) / tile > 65536) {
       delete b;
@@ -946,9 +949,12 @@ int mpdata_batch_create(int nprob, const mpdata_problem* probs, int ih, int iord
       b->gv[p] = (iord >= 2 && members[o] >= 2 && b->fzi[p] < 0) ? forms[o] : 0;
     }
   }
+  // velocity scratch: the tile kernels' (a group's problems share one grid, so all of
+  // them run on the fused kernels or none)
   for (int p = 0; p < nprob; p++)
     if (b->owner[p] == p) {
       b->voff[p] = off;
+      if (b->fzi[p] >= 0) continue;
       off += (size_t)(NVEL + ((b->gv[p] & 1) ? NGVEL : 0) + ((b->gv[p] & 2) ? NGVS : 0)) * b->ncell[p];
     }
   for (int p = 0; p < nprob; p++) b->voff[p] = b->voff[b->owner[p]];

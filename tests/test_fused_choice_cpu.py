@@ -48,6 +48,16 @@ def test_kernels_by_how_a_grid_fills_their_tiles(native_lib, monkeypatch, count,
     assert classes(native_lib, [size] * count, ibc, gauge) == [want] * count
 
 
+@pytest.mark.parametrize("size,ibc,gauge,want", [
+    ((2, 100000, 5000), OPEN, 1, NONE),     # a wide arena of 312 GB, 76 GB of stage scratch
+    ((2, 100000, 5000), PER, 1, NARROW),
+    ((8, 200000, 300), PER, 0, NONE),
+    ((4096, 4096, 100), OPEN, 0, STD)])
+def test_an_arena_takes_no_more_than_the_stage_scratch(native_lib, monkeypatch, size, ibc, gauge, want):
+    monkeypatch.delenv("MPDATA_FUSED", raising=False)
+    assert classes(native_lib, [size], ibc, gauge) == [want]
+
+
 def test_a_mixed_batch_is_judged_by_all_its_cells(native_lib, monkeypatch):
     """A few narrow domains among large ones share the large ones' launch."""
     monkeypatch.delenv("MPDATA_FUSED", raising=False)

@@ -105,3 +105,15 @@ def test_thin_walls_take_the_stage_kernels(M, oracle):
         got, n, _ = run(M, f, gauge, 2, 2)
         assert n == 2 * 5  # upwind, pseudo, bounds, limit, update
         same_bits(W.interior(got), oracle_steps(oracle, f, gauge, 2, 2))
+
+
+def test_fused_batch_takes_no_velocity_scratch(M):
+    """A batch on the fused kernels needs its fields' scratch alone (15 fields each),
+    not the tile kernels' velocity terms (4 more)."""
+    import torch
+    n, m, l = 256, 256, 64
+    free0 = torch.cuda.mem_get_info()[0]
+    b = M.Batch([dict(np=n, mp=m, lp=l)], iord=2, precision=32)
+    fields = (free0 - torch.cuda.mem_get_info()[0]) / (4.0 * n * m * l)
+    b.close()
+    assert fields < 16.5, fields
