@@ -616,41 +616,20 @@ __global__ void KA_LB_PSEUDO ka_pseudo(const Prob<R> P, const AdjArr<R> A) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z + 1;
   const bool win = warp_interior(P.g, i, j, k);
-  // every pair sum stored (pairs 2): full warps at a boundary read them too
-  bool pin = false;
-  if (!win && P.pairs == 2) pin = warp_on_grid(P.g, i, j);
+  // every pair sum is stored: full warps at a boundary read them too
+  const bool pin = !win && warp_on_grid(P.g, i, j);
   if (i > P.g.np || j > P.g.mp) return;
-  if (!win) {
-    if (pin) {
-      if (warp_unit_faces(P, i, j, k))
-        ka_pseudo_cell<R, AIN, false, true, true, true>(P, A, i, j, k);
-      else
-        ka_pseudo_cell<R, AIN, false, false, true, true>(P, A, i, j, k);
-      return;
-    }
+  if (pin) {
+    if (warp_unit_faces(P, i, j, k))
+      ka_pseudo_cell<R, AIN, false, true, true, true>(P, A, i, j, k);
+    else
+      ka_pseudo_cell<R, AIN, false, false, true, true>(P, A, i, j, k);
+  } else if (!win) {
     ka_pseudo_cell<R, AIN, false>(P, A, i, j, k);
-  } else if constexpr (sizeof(R) == 8) {
-    const bool unit = warp_unit_faces(P, i, j, k);
-    if (P.pairs == 2) {
-      if (unit)
-        ka_pseudo_cell<R, AIN, true, true, true, true>(P, A, i, j, k);
-      else
-        ka_pseudo_cell<R, AIN, true, false, true, true>(P, A, i, j, k);
-    } else if (P.pairs) {
-      if (unit)
-        ka_pseudo_cell<R, AIN, true, true, true>(P, A, i, j, k);
-      else
-        ka_pseudo_cell<R, AIN, true, false, true>(P, A, i, j, k);
-    } else {
-      if (unit)
-        ka_pseudo_cell<R, AIN, true, true>(P, A, i, j, k);
-      else
-        ka_pseudo_cell<R, AIN, true>(P, A, i, j, k);
-    }
-  } else if (P.pairs == 2) {  // FP32: the stored pairs save issue slots
-    ka_pseudo_cell<R, AIN, true, false, true, true>(P, A, i, j, k);
+  } else if (warp_unit_faces(P, i, j, k)) {  // FP64
+    ka_pseudo_cell<R, AIN, true, true, true, true>(P, A, i, j, k);
   } else {
-    ka_pseudo_cell<R, AIN, true>(P, A, i, j, k);
+    ka_pseudo_cell<R, AIN, true, false, true, true>(P, A, i, j, k);
   }
 }
 
@@ -1223,11 +1202,6 @@ __global__ void __launch_bounds__(128, KfPseudoMinBlocks<R>::v) kf_pseudo(const 
         pseudo_body<R, AIN, true, true, true, false, true, true>(P, i, j, k);
       else
         pseudo_body<R, AIN, true, false, true, false, true, true>(P, i, j, k);
-    } else if (P.pairs) {
-      if (unit)
-        pseudo_body<R, AIN, true, true, true>(P, i, j, k);
-      else
-        pseudo_body<R, AIN, true, false, true>(P, i, j, k);
     } else {
       if (unit)
         pseudo_body<R, AIN, true, true>(P, i, j, k);
@@ -1513,18 +1487,15 @@ int reverse_passes(const Prob<R>& P, const AdjPlan<R>& A, int nonos, bool kept, 
       }
       // the pass's cp/cn/q records are dead once the reverse bounds ran:
       // they take the pair sums of its input field, and the workspace's
-      // f1..f3 the velocity pairs (FP64)
+      // f1..f3 the velocity pairs
       Prob<R> Qp = Q;
-      Qp.pairs = 2;
-      if (Qp.pairs) {
-        Qp.f1 = P.f1;
-        Qp.f2 = P.f2;
-        Qp.f3 = P.f3;
-        if (kept) pairs_in_lf(&Qp, A);
-        else if (t == 0) chain_launch(kf_pairs<R, true, true>, grd, blk, 0, s, Qp);
-        else chain_launch(kf_pairs<R, false, true>, grd, blk, 0, s, Qp);
-        n += kept ? 0 : 1;
-      }
+      Qp.f1 = P.f1;
+      Qp.f2 = P.f2;
+      Qp.f3 = P.f3;
+      if (kept) pairs_in_lf(&Qp, A);
+      else if (t == 0) chain_launch(kf_pairs<R, true, true>, grd, blk, 0, s, Qp);
+      else chain_launch(kf_pairs<R, false, true>, grd, blk, 0, s, Qp);
+      n += kept ? 0 : 1;
       if (sizeof(R) == 4 && g.bx && g.by && g.bz) {
         if constexpr (sizeof(R) == 4) {
           if (t == 0) chain_launch(ka_cross<R, true>, grd, blk, 0, s, Qp, a);

@@ -129,22 +129,26 @@ __global__ void __launch_bounds__(256) kb_copy(BATCH_ARGS) {
   BATCH_TILE(B)
 #undef B
 }
+// P.pairs: FP64 gauge problems alone, so the pair variants are the gauge form's.
 template <class R, bool AIN>
 __device__ __forceinline__ void pseudo_dispatch(const Prob<R>& P, int i, int j, int k, bool win, bool pin) {
   if constexpr (AIN) {
     // first pass of a velocity group: its form's velocity-only terms are precomputed
     if (win && (P.stdf ? (P.gv & 2) : (P.gv & 1))) {
-      if (warp_unit_faces(P, i, j, k)) {
-        if (P.pairs)
-          pseudo_body<R, AIN, true, true, true, true, false>(P, i, j, k);
-        else
-          pseudo_body<R, AIN, true, true, false, true, false>(P, i, j, k);
-      } else {
-        if (P.pairs)
-          pseudo_body<R, AIN, true, false, true, true, false>(P, i, j, k);
-        else
-          pseudo_body<R, AIN, true, false, false, true, false>(P, i, j, k);
+      const bool unit = warp_unit_faces(P, i, j, k);
+      if constexpr (sizeof(R) == 8) {
+        if (P.pairs) {
+          if (unit)
+            pseudo_form<R, false, AIN, true, true, true, true, false>(P, i, j, k);
+          else
+            pseudo_form<R, false, AIN, true, false, true, true, false>(P, i, j, k);
+          return;
+        }
       }
+      if (unit)
+        pseudo_body<R, AIN, true, true, false, true, false>(P, i, j, k);
+      else
+        pseudo_body<R, AIN, true, false, false, true, false>(P, i, j, k);
       return;
     }
   }
@@ -152,9 +156,9 @@ __device__ __forceinline__ void pseudo_dispatch(const Prob<R>& P, int i, int j, 
     if constexpr (sizeof(R) == 8) {
       if (pin) {  // a full warp at a boundary: the stored pairs through the boundary maps
         if (warp_unit_faces(P, i, j, k))
-          pseudo_body<R, AIN, false, true, true, false, false, true>(P, i, j, k);
+          pseudo_form<R, false, AIN, false, true, true, false, false, true>(P, i, j, k);
         else
-          pseudo_body<R, AIN, false, false, true, false, false, true>(P, i, j, k);
+          pseudo_form<R, false, AIN, false, false, true, false, false, true>(P, i, j, k);
         return;
       }
     }
@@ -163,9 +167,9 @@ __device__ __forceinline__ void pseudo_dispatch(const Prob<R>& P, int i, int j, 
     const bool unit = warp_unit_faces(P, i, j, k);
     if (P.pairs) {  // outside the group branch above, the velocity pairs are stored too
       if (unit)
-        pseudo_body<R, AIN, true, true, true, false, false, true>(P, i, j, k);
+        pseudo_form<R, false, AIN, true, true, true, false, false, true>(P, i, j, k);
       else
-        pseudo_body<R, AIN, true, false, true, false, false, true>(P, i, j, k);
+        pseudo_form<R, false, AIN, true, false, true, false, false, true>(P, i, j, k);
     } else {
       if (unit)
         pseudo_body<R, AIN, true, true, false, false, false>(P, i, j, k);
