@@ -21,7 +21,7 @@ INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
                      "-I" + INCLUDE, "-I" + CSRC]
-# Extra nvcc flags for tuning sweeps (e.g. "-DMPDATA_FZ_TY=16"); a build with
+# Extra nvcc flags for tuning sweeps (e.g. "-DMPDATA_MINB_UPWIND_F64=7"); a build with
 # them is never up to date with a default build.
 EXTRA = os.environ.get("MPDATA_NVCC_EXTRA", "").split()
 

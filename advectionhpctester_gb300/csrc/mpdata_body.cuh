@@ -25,9 +25,9 @@ struct Prob {
   int stdf;     // 1 = standard form (t_adv=2), 0 = infinite gauge (t_adv=1)
   int own_vel;  // 1 = this problem writes the velocity-derived scratch (hinv, hm*)
   int rho;      // density step of mpdata3d_rho_gauge_gpubc: no rhr, upwind fluxes kept
-  int pairs;    // gauge pseudo-velocity: 1 = pair sums of xant in cp, cn, q
-                // (k_pairs); 2 = also the pass velocities' cell-centred pairs
-                // in f1..f3, which lets full warps at a boundary take the pair path
+  int pairs;    // FP64 pseudo-velocity: 1 = pair sums of xant (of |xant| in the
+                // standard form) in cp, cn, q (k_pairs); 2 = also the pass velocities'
+                // cell-centred pairs, in f1..f3 (standard form: w1..w3)
   int gv;       // batch velocity group: the velocity-only terms of the first
                 // pass's pseudo-velocities, stored by the group owner's upwind:
                 // bit 0 the gauge form's (gvf), bit 1 the standard form's (gvs)
@@ -354,15 +354,16 @@ __device__ __forceinline__ void upwind_body(const Prob<R>& P, int i, int j, int 
 // Each cell computes its lower faces.  AIN: the first corrective pass, whose
 // "a" velocities are the caller's Courant numbers; later passes use the
 // previous pass's limited velocities w1..w3.  U: the three face reciprocal
-// densities of every cell of the warp are exactly 1 (warp_unit_faces).  PS
-// (gauge, interior warps): the pair sums of xant the rat4 terms start with
-// are read from cp, cn and q, where k_pairs stored them.  GV (gauge, first
-// pass, interior warps of a batch velocity group): the velocity-only terms
-// are read from gvf (velgroup_body).  PV (gauge, with PS): the velocities'
-// cell-centred pairs of the 4-face sums are read from f1..f3, where k_pairs
-// stored them.  Without IN (a full warp at a boundary), PS reads the xant
-// pairs through the xant halo maps and PV the velocity pairs through the
-// face maps, so each stored pair is the sum the generic body forms there.
+// densities of every cell of the warp are exactly 1 (warp_unit_faces).  PS: the
+// pair sums of xant the rat4 terms start with (in the standard form of |xant|,
+// with which its quotients' terms start) are read from cp, cn and q, where
+// k_pairs stored them.  GV (first pass, interior warps of a batch velocity group):
+// the velocity-only terms are read from gvf or gvs (velgroup_body).  PV (with PS):
+// the velocities' cell-centred pairs of the 4-face sums are read where k_pairs
+// stored them, f1..f3 in the gauge form, w1..w3 in the standard form (its first
+// pass alone).  Without IN (a warp at a boundary), PS reads the xant pairs through
+// the xant halo maps and PV the velocity pairs through the face maps, so each
+// stored pair is the sum the generic body forms there.
 template <class R, bool STD, bool AIN, bool IN = false, bool U = false, bool PS = false, bool GV = false,
           bool DEFER = true, bool PV = false>
 __device__ __forceinline__ void pseudo_form(const Prob<R>& P, int i, int j, int k) {

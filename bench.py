@@ -39,14 +39,14 @@ UNIT = "Gcell-steps/s"
 # Algorithmic (compulsory) device bytes per cell per launch of each stage:
 # every array a kernel must read or write, once.  Units: elements per cell.
 #   upwind   r psi u1..3 h rhr                w xant hinv hmx hmy hmz   11
-#   pairs    r xant                           w Sx Sy Sz                 4 (FP64 gauge only)
+#   pairs    r xant                           w Sx Sy Sz                 4 (FP64)
 #   pseudo   r xant a1..3 hm1..3 (+Sx Sy Sz)  w v1..3 (+f1..3 std)      10, 13 FP64 gauge (13 std)
 #   bounds   r xant psi|mx,mn h rhr F1..3     w q cp cn (+mx mn)        10..13
 #   limit    r cp cn v1..3 (+xant q)          w w1..3 (+f1..3)          8 (13 std)
 #   update   r q rhr h|hinv F1..3             w out                     7
 #   predictor level  r o0 x3 o2 x3 h  w o1 x3 o2 x3 (the level roll)     13
 #   predictor cgrid  r o1 x3          w u1..3                             6
-# The fused single-precision step (periodic gauge grids):
+# The fused single-precision step (limiter, iord >= 2):
 #   fused_upwind_pseudo  r psi u1..3 h rhr     w x_in xant v1..3           11
 #   fused_pseudo         r x w1..3             w v1..3                      7
 #   fused_limit_update   r x x_in|mx,mn v1..3  w x (w1..3) (mx mn)        9..12
