@@ -901,7 +901,7 @@ void narrow_kchunk(const Geo* g, int n, int* kchunk) {
       rest += (g[p].mp + TY2 - 1) / TY2 * steps;
       longest = std::max(longest, kc + START);
     }
-    const double resident = 152.0 * longest;
+    const double resident = num_sms() * longest;
     return (rounds(up / (resident * Tl<TY_UP>::MINB)) + rounds(rest / (resident * Tl<TY2>::MINB))) * longest;
   };
   // the candidates that split the longest problem evenly

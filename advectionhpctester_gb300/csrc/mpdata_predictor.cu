@@ -192,19 +192,6 @@ __global__ void __launch_bounds__(128) k_pred_cgrid(Geo g, long lev, R* ox, R* o
   }
 }
 
-// SMs of the current device (queried once).
-int num_sms() {
-  static int n = 0;
-  if (n < 1) {
-    int dev = 0, v = 0;
-    n = (cudaGetDevice(&dev) == cudaSuccess &&
-         cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            ? v
-            : 152;
-  }
-  return n;
-}
-
 // The C-grid averaging of level 1 (velprdA_to_C, module_velprd.f90:197-361)
 // as a march up the z columns: each thread owns the (i, j) column of a chunk
 // of planes and keeps the level-1 value of the plane below in a register, so

@@ -218,6 +218,20 @@ __global__ void __launch_bounds__(128) k_rho_out(const Prob<R> P) {
   rho_out_body<R, LINER>(P, i, j, k);
 }
 
+// SMs of the current device (queried once; without a device those of the GB300 that the
+// dispatch rules were measured on).
+int num_sms() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
+      return v;
+    cudaGetLastError();
+    return 152;
+  }();
+  return n;
+}
+
 // ---- launch accounting ---------------------------------------------------
 static unsigned long long g_launches = 0;
 unsigned long long launch_count() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }

@@ -150,6 +150,7 @@ int run_rho_out_adjoint(const Prob<R>& P, const Arr<R>& out, const Arr<R>& lxc, 
                         const Arr<R>& g_pexe, cudaStream_t s);
 
 unsigned long long launch_count();
+int num_sms();
 void add_launches(int n);
 
 }  // namespace mpdata
