@@ -82,6 +82,7 @@ def chunks(lib, sizes, cls, ibc=PER):
     (2, (80, 32, 32), WALL, 3),        # 47 us, 61 with the 1 plane of the rule for uneven lists
     (6, (80, 32, 32), PERIODIC, 4),    # 56 : 76
     (24, (48, 48, 48), STD, 16),       # 246 : 303
+    (200, (40, 40, 40), PERIODIC, 20),  # 1.02 ms; a long launch keeps the average
     (64, (32, 32, 32), NARROW, 16), (6, (32, 32, 32), NARROW, 3)])
 def test_equal_grids_count_rounds(native_lib, monkeypatch, count, size, cls, want):
     monkeypatch.delenv("MPDATA_FUSED_KCHUNK", raising=False)
